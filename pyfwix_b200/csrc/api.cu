@@ -270,6 +270,9 @@ fwix_status phase_factors(fwix_plan* p, int iz, SpecArgs& a, cudaStream_t s) {
   float2* dst = p->pcache + slot * p->pdepth();
   a.ptab_nx = p->pq_nx();
   a.ptab_ny = p->pq_ny();
+  const bool kx_fast = !fwix::fast_length(p->d.NY) && fwix::resident_length(p->d.NY);
+  a.ptab_sx = kx_fast ? 1 : a.ptab_ny;
+  a.ptab_sy = kx_fast ? a.ptab_nx : 1;
   if (p->pslot_iz[slot] != iz) {
     SpecArgs b = a;
     b.sref = p->sref + (long long)iz * p->desc.nref * p->d.nw;
@@ -393,7 +396,7 @@ fwix_status smooth_chunk(fwix_plan* p, int iz, int mode, SpecArgs a, cudaStream_
   FWIX_TRY(cu(fwix::row_forward(a, fwix::W_TAPER, s), "smooth row pass"));
   FWIX_TRY(cu(fwix::col_type_a(a, fwix::Q_PS_FWD, s), "smooth column pass"));
   if (mode == kSmoothPair) {
-    if (fwix::fast_length(p->d.NX))
+    if (fwix::resident_length(p->d.NX))
       return cu(fwix::row_inverse(a, fwix::W_SMOOTH_PAIR, 0, s), "smooth pair inverse row pass");
     FWIX_TRY(cu(fwix::row_inverse(a, fwix::W_SMOOTH, 0, s), "smooth inverse row pass"));
     a.out = a.out2;
@@ -438,7 +441,7 @@ fwix_status do_scatter(fwix_plan* p, int iz, int adjoint, const float2* in, floa
     FWIX_TRY(cu(fwix::launch_scat_table(a0, p->scat_tab, s), "scatter weights"));
     a0.scat_tab = p->scat_tab;
   }
-  if (adjoint && p->desc.taylor >= 1 && fwix::fast_length(p->d.NX) && fwix::fast_length(p->d.NY)) {
+  if (adjoint && p->desc.taylor >= 1 && fwix::resident_length(p->d.NX) && fwix::resident_length(p->d.NY)) {
     // the zeroth term's filter is the identity: conj(W_0) d is added by the inverse
     // row pass, and only orders 1 .. taylor go through the transforms.  (The
     // forward keeps the zeroth term in the transforms: measured on B200, adding

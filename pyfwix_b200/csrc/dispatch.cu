@@ -1,5 +1,6 @@
 // use the register-resident passes of fast.cuh; every other supported length uses
 // the per-warp Stockham passes of spectral.cu.  Rows dispatch on NX, columns on NY.
+#include "flex.h"
 #include "internal.h"
 
 #define FWIX_FAST_DECL(TAG)                                                                            \
@@ -42,6 +43,8 @@ bool fast_length(int n) {
   }
 }
 
+bool resident_length(int n) { return fast_length(n) || flex::has_plan(n); }
+
 cudaError_t row_forward(const SpecArgs& a, int pre, cudaStream_t s) {
   switch (a.d.NX) {
     case 64: return fast::row_forward_64(a, pre, s);
@@ -54,7 +57,7 @@ cudaError_t row_forward(const SpecArgs& a, int pre, cudaStream_t s) {
     case 384: return fast::row_forward_384(a, pre, s);
     case 512: return fast::row_forward_512(a, pre, s);
     case 640: return fast::row_forward_640(a, pre, s);
-    default: return generic_row_forward(a, pre, s);
+    default: return flex::has_plan(a.d.NX) ? flex::row_forward(a, pre, s) : generic_row_forward(a, pre, s);
   }
 }
 
@@ -70,7 +73,7 @@ cudaError_t row_inverse(const SpecArgs& a, int post, int post_taper, cudaStream_
     case 384: return fast::row_inverse_384(a, post, post_taper, s);
     case 512: return fast::row_inverse_512(a, post, post_taper, s);
     case 640: return fast::row_inverse_640(a, post, post_taper, s);
-    default: return generic_row_inverse(a, post, post_taper, s);
+    default: return flex::has_plan(a.d.NX) ? flex::row_inverse(a, post, post_taper, s) : generic_row_inverse(a, post, post_taper, s);
   }
 }
 
@@ -86,7 +89,7 @@ cudaError_t col_type_a(const SpecArgs& a, int qmode, cudaStream_t s) {
     case 384: return fast::col_type_a_384(a, qmode, s);
     case 512: return fast::col_type_a_512(a, qmode, s);
     case 640: return fast::col_type_a_640(a, qmode, s);
-    default: return generic_col_type_a(a, qmode, s);
+    default: return flex::has_plan(a.d.NY) ? flex::col_type_a(a, qmode, s) : generic_col_type_a(a, qmode, s);
   }
 }
 
@@ -102,7 +105,7 @@ cudaError_t col_type_b(const SpecArgs& a, int qmode, cudaStream_t s) {
     case 384: return fast::col_type_b_384(a, qmode, s);
     case 512: return fast::col_type_b_512(a, qmode, s);
     case 640: return fast::col_type_b_640(a, qmode, s);
-    default: return generic_col_type_b(a, qmode, s);
+    default: return flex::has_plan(a.d.NY) ? flex::col_type_b(a, qmode, s) : generic_col_type_b(a, qmode, s);
   }
 }
 
@@ -119,7 +122,7 @@ cudaError_t col_fft(const SpecArgs& a, int inverse, const float2* in, float2* ou
     case 384: return fast::col_fft_384(a, inverse, in, out, add, scale, s);
     case 512: return fast::col_fft_512(a, inverse, in, out, add, scale, s);
     case 640: return fast::col_fft_640(a, inverse, in, out, add, scale, s);
-    default: return generic_col_fft(a, inverse, in, out, add, scale, s);
+    default: return flex::has_plan(a.d.NY) ? flex::col_fft(a, inverse, in, out, add, scale, s) : generic_col_fft(a, inverse, in, out, add, scale, s);
   }
 }
 

@@ -35,6 +35,9 @@ __device__ __forceinline__ float2 cmul_conj(float2 a, float2 b) {  // a * conj(b
 __device__ __forceinline__ float2 cadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ float2 csub(float2 a, float2 b) { return __fadd2_rn(a, make_float2(-b.x, -b.y)); }
 __device__ __forceinline__ float2 cscale(float2 a, float s) { return __fmul2_rn(a, make_float2(s, s)); }
+__device__ __forceinline__ float2 cfma(float2 a, float s, float2 b) {  // a s + b
+  return __ffma2_rn(a, make_float2(s, s), b);
+}
 #else
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
   return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
@@ -45,6 +48,9 @@ __device__ __forceinline__ float2 cmul_conj(float2 a, float2 b) {  // a * conj(b
 __device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
 __device__ __forceinline__ float2 cscale(float2 a, float s) { return make_float2(a.x * s, a.y * s); }
+__device__ __forceinline__ float2 cfma(float2 a, float s, float2 b) {  // a s + b
+  return make_float2(fmaf(a.x, s, b.x), fmaf(a.y, s, b.y));
+}
 #endif
 __device__ __forceinline__ float2 cconj(float2 a) { return make_float2(a.x, -a.y); }
 // multiply by -i (forward) or +i (inverse)
@@ -133,7 +139,7 @@ struct Dft<3, INV> {
     const float s3 = 0.86602540378443864676f;
     float2 t = cadd(v[1], v[2]);
     float2 u = rot90<INV>(cscale(csub(v[1], v[2]), s3));  // -+ i s3 (v1 - v2)
-    float2 m = make_float2(v[0].x - 0.5f * t.x, v[0].y - 0.5f * t.y);
+    float2 m = cfma(t, -0.5f, v[0]);
     v[0] = cadd(v[0], t);
     v[1] = cadd(m, u);
     v[2] = csub(m, u);
@@ -149,10 +155,10 @@ struct Dft<5, INV> {
     const float s2 = 0.58778525229247312917f;   // sin(4 pi / 5)
     float2 t1 = cadd(v[1], v[4]), t2 = cadd(v[2], v[3]);
     float2 u1 = csub(v[1], v[4]), u2 = csub(v[2], v[3]);
-    float2 a1 = make_float2(v[0].x + c1 * t1.x + c2 * t2.x, v[0].y + c1 * t1.y + c2 * t2.y);
-    float2 a2 = make_float2(v[0].x + c2 * t1.x + c1 * t2.x, v[0].y + c2 * t1.y + c1 * t2.y);
-    float2 b1 = rot90<INV>(make_float2(s1 * u1.x + s2 * u2.x, s1 * u1.y + s2 * u2.y));
-    float2 b2 = rot90<INV>(make_float2(s2 * u1.x - s1 * u2.x, s2 * u1.y - s1 * u2.y));
+    float2 a1 = cfma(t2, c2, cfma(t1, c1, v[0]));
+    float2 a2 = cfma(t2, c1, cfma(t1, c2, v[0]));
+    float2 b1 = rot90<INV>(cfma(u2, s2, cscale(u1, s1)));
+    float2 b2 = rot90<INV>(cfma(u2, -s1, cscale(u1, s2)));
     v[0] = cadd(v[0], cadd(t1, t2));
     v[1] = cadd(a1, b1);
     v[4] = csub(a1, b1);
@@ -199,41 +205,6 @@ struct Dft<16, INV> {
   }
 };
 
-// Radix 4 N2 for N2 = 3, 5 by the prime-factor (Good-Thomas) mapping, which needs
-// no twiddles between the two transforms: input n = (N2 n1 + 4 n2) mod N, radix-N2
-// transforms over n2, radix-4 transforms over n1, output k = k1 (mod 4),
-// k = k2 (mod N2), i.e. k = (A k1 + B k2) mod N with A = N2 (N2^-1 mod 4) and
-// B = 4 (4^-1 mod N2): (9, 4) for 12, (5, 16) for 20.
-template <int N2, int A, int B, bool INV>
-__device__ __forceinline__ void dft_pfa4(float2 (&v)[4 * N2]) {
-  constexpr int N = 4 * N2;
-  float2 y[4][N2];
-#pragma unroll
-  for (int n1 = 0; n1 < 4; ++n1) {
-    float2 u[N2];
-#pragma unroll
-    for (int n2 = 0; n2 < N2; ++n2) u[n2] = v[(N2 * n1 + 4 * n2) % N];
-    Dft<N2, INV>::run(u);
-#pragma unroll
-    for (int k2 = 0; k2 < N2; ++k2) y[n1][k2] = u[k2];
-  }
-#pragma unroll
-  for (int k2 = 0; k2 < N2; ++k2) {
-    float2 u[4] = {y[0][k2], y[1][k2], y[2][k2], y[3][k2]};
-    Dft<4, INV>::run(u);
-#pragma unroll
-    for (int k1 = 0; k1 < 4; ++k1) v[(A * k1 + B * k2) % N] = u[k1];
-  }
-}
-template <bool INV>
-struct Dft<12, INV> {
-  static __device__ __forceinline__ void run(float2 (&v)[12]) { dft_pfa4<3, 9, 4, INV>(v); }
-};
-template <bool INV>
-struct Dft<20, INV> {
-  static __device__ __forceinline__ void run(float2 (&v)[20]) { dft_pfa4<5, 5, 16, INV>(v); }
-};
-
 // Radix 7 from the symmetric pair form y_m = v0 + sum_k cos(2 pi k m/7) t_k -+
 // i sum_k sin(2 pi k m/7) u_k with t_k = v_k + v_{7-k}, u_k = v_k - v_{7-k}.
 template <bool INV>
@@ -253,18 +224,111 @@ struct Dft<7, INV> {
     v[0] = cadd(v0, cadd(t[1], cadd(t[2], t[3])));
 #pragma unroll
     for (int m = 1; m <= 3; ++m) {
-      float2 a = v0, b = make_float2(0.f, 0.f);
+      float2 a = cfma(t[1], C[m], v0), b = cscale(u[1], S[m]);
 #pragma unroll
-      for (int k = 1; k <= 3; ++k) {
+      for (int k = 2; k <= 3; ++k) {
         const int j = (k * m) % 7;
-        a = make_float2(a.x + C[j] * t[k].x, a.y + C[j] * t[k].y);
-        b = make_float2(b.x + S[j] * u[k].x, b.y + S[j] * u[k].y);
+        a = cfma(t[k], C[j], a);
+        b = cfma(u[k], S[j], b);
       }
       const float2 rb = rot90<INV>(b);
       v[m] = cadd(a, rb);
       v[7 - m] = csub(a, rb);
     }
   }
+};
+
+// Radix N1 N2 with coprime factors by the prime-factor (Good-Thomas) mapping, which
+// needs no twiddles between the two transforms: input n = (N2 n1 + N1 n2) mod N,
+// radix-N2 transforms over n2, radix-N1 transforms over n1, output k = k1 (mod N1),
+// k = k2 (mod N2), i.e. k = (A k1 + B k2) mod N with A = N2 (N2^-1 mod N1) and
+// B = N1 (N1^-1 mod N2).
+constexpr int mod_inverse(int v, int m) {
+  for (int i = 1; i < m; ++i)
+    if ((v * i) % m == 1) return i;
+  return 1;
+}
+template <int N1, int N2, bool INV>
+__device__ __forceinline__ void dft_pfa(float2 (&v)[N1 * N2]) {
+  constexpr int N = N1 * N2, A = N2 * mod_inverse(N2 % N1, N1), B = N1 * mod_inverse(N1 % N2, N2);
+  float2 y[N1][N2];
+#pragma unroll
+  for (int n1 = 0; n1 < N1; ++n1) {
+    float2 u[N2];
+#pragma unroll
+    for (int n2 = 0; n2 < N2; ++n2) u[n2] = v[(N2 * n1 + N1 * n2) % N];
+    Dft<N2, INV>::run(u);
+#pragma unroll
+    for (int k2 = 0; k2 < N2; ++k2) y[n1][k2] = u[k2];
+  }
+#pragma unroll
+  for (int k2 = 0; k2 < N2; ++k2) {
+    float2 u[N1];
+#pragma unroll
+    for (int n1 = 0; n1 < N1; ++n1) u[n1] = y[n1][k2];
+    Dft<N1, INV>::run(u);
+#pragma unroll
+    for (int k1 = 0; k1 < N1; ++k1) v[(A * k1 + B * k2) % N] = u[k1];
+  }
+}
+
+// Radix 9 as 3 x 3: n = 3 n1 + n2, k = k1 + 3 k2; radix-3 transforms over n1,
+// twiddles W9^(n2 k1), radix-3 transforms over n2.
+template <bool INV>
+struct Dft<9, INV> {
+  static __device__ __forceinline__ void run(float2 (&v)[9]) {
+    const float c1 = 0.76604444311897803520f, s1 = 0.64278760968653932632f;   // cos, sin 40 degrees
+    const float c2 = 0.17364817766693034885f, s2 = 0.98480775301220805937f;   // 80
+    const float c4 = -0.93969262078590838405f, s4 = 0.34202014332566873304f;  // 160
+    float2 y[3][3];
+#pragma unroll
+    for (int n2 = 0; n2 < 3; ++n2) {
+      float2 u[3] = {v[n2], v[3 + n2], v[6 + n2]};
+      Dft<3, INV>::run(u);
+#pragma unroll
+      for (int k1 = 0; k1 < 3; ++k1) y[n2][k1] = u[k1];
+    }
+    y[1][1] = tw16<INV>(y[1][1], c1, s1);
+    y[1][2] = tw16<INV>(y[1][2], c2, s2);
+    y[2][1] = tw16<INV>(y[2][1], c2, s2);
+    y[2][2] = tw16<INV>(y[2][2], c4, s4);
+#pragma unroll
+    for (int k1 = 0; k1 < 3; ++k1) {
+      float2 u[3] = {y[0][k1], y[1][k1], y[2][k1]};
+      Dft<3, INV>::run(u);
+#pragma unroll
+      for (int k2 = 0; k2 < 3; ++k2) v[k1 + 3 * k2] = u[k2];
+    }
+  }
+};
+
+template <bool INV>
+struct Dft<6, INV> {
+  static __device__ __forceinline__ void run(float2 (&v)[6]) { dft_pfa<2, 3, INV>(v); }
+};
+template <bool INV>
+struct Dft<10, INV> {
+  static __device__ __forceinline__ void run(float2 (&v)[10]) { dft_pfa<2, 5, INV>(v); }
+};
+template <bool INV>
+struct Dft<12, INV> {
+  static __device__ __forceinline__ void run(float2 (&v)[12]) { dft_pfa<4, 3, INV>(v); }
+};
+template <bool INV>
+struct Dft<14, INV> {
+  static __device__ __forceinline__ void run(float2 (&v)[14]) { dft_pfa<2, 7, INV>(v); }
+};
+template <bool INV>
+struct Dft<15, INV> {
+  static __device__ __forceinline__ void run(float2 (&v)[15]) { dft_pfa<3, 5, INV>(v); }
+};
+template <bool INV>
+struct Dft<18, INV> {
+  static __device__ __forceinline__ void run(float2 (&v)[18]) { dft_pfa<2, 9, INV>(v); }
+};
+template <bool INV>
+struct Dft<20, INV> {
+  static __device__ __forceinline__ void run(float2 (&v)[20]) { dft_pfa<4, 5, INV>(v); }
 };
 
 // One Stockham pass of radix R over a line of n elements at element stride `st`.

@@ -80,11 +80,13 @@ struct SpecArgs {
   const float2* image; // imaging-condition image, (iw, y, x) at image[iw*img_w + y*nx + x] (W_IC)
   long long img_w;     // ny*nx, or 0 for one image shared by every frequency
   // cached forward phase factors of this depth (x norm), element (ref, iw, |kx|, |ky|)
-  // at ptab[((ref*nw + iw)*ptab_nx + kxq)*ptab_ny + kyq], kxq = min(x, NX-x),
-  // kyq = min(y, NY-y); ptab_nx = NX/2 + 1, ptab_ny = NY/2 + 1 rounded up to even
-  // (16-byte rows for TMA); NULL means evaluate the factors in the kernel
+  // at ptab[(ref*nw + iw)*ptab_nx*ptab_ny + kxq*ptab_sx + kyq*ptab_sy], kxq =
+  // min(x, NX-x), kyq = min(y, NY-y); ptab_nx = NX/2 + 1, ptab_ny = NY/2 + 1 rounded
+  // up to even (16-byte rows for TMA).  ky runs fastest for the columns whose lanes
+  // run along ky (compile-time plans), kx for those whose lanes run across the
+  // columns (flex.cuh).  NULL means evaluate the factors in the kernel
   const float2* ptab;
-  int ptab_nx, ptab_ny;
+  int ptab_nx, ptab_ny, ptab_sx, ptab_sy;
   // smooth step: padded local slowness [NY][NX] and the sorted real reference
   // slownesses [sm_n] of this depth
   const float* sm_s;
@@ -143,9 +145,13 @@ struct SpecArgs {
 };
 
 // Spectral passes (dispatch.cu: register-resident passes for lengths with a
-// compile-time plan, else the generic per-warp passes of spectral.cu).  Each
+// compile-time plan (fast.cuh) or a run-time one (flex.cuh), the generic per-warp
+// passes of spectral.cu for the few lengths with neither).  Each
 // returns a CUDA error code.
 bool fast_length(int n);
+// Whether lines of n samples run register-resident passes (a compile-time plan or
+// one of flex.h): these take the paired smooth weights and the direct Born term.
+bool resident_length(int n);
 cudaError_t row_forward(const SpecArgs& a, int pre, cudaStream_t s);      // in -> t1[0..nterm)
 cudaError_t row_inverse(const SpecArgs& a, int post, int post_taper, cudaStream_t s);  // t2 -> out
 cudaError_t col_type_a(const SpecArgs& a, int qmode, cudaStream_t s);     // t1[0] -> t2[0..nterm)

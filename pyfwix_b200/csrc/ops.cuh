@@ -171,7 +171,7 @@ __device__ __forceinline__ float2 qmult(const SpecArgs& a, int t, int iw, int x,
   const float w2 = a.w2[iw];
   if ((QM == Q_PS_FWD || QM == Q_PS_ADJ) && a.ptab) {
     const int kxq = min(x, a.d.NX - x), kyq = min(y, a.d.NY - y);
-    const float2 P = a.ptab[(((long long)t * a.d.nw + iw) * a.ptab_nx + kxq) * a.ptab_ny + kyq];
+    const float2 P = a.ptab[((long long)t * a.d.nw + iw) * a.ptab_nx * a.ptab_ny + kxq * a.ptab_sx + kyq * a.ptab_sy];
     if (QM == Q_PS_FWD) return P;
     // adjoint factor: conj(P), or P itself where the reference flips Re (b > 0)
     const float bb = w2 * (sr.y - a.eps * sr.x);

@@ -463,10 +463,13 @@ __global__ void k_phase_table(const SpecArgs a, float2* dst) {
   b.ptab = nullptr;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {
-    const int kyq = (int)(i % a.ptab_ny);
-    long long q = i / a.ptab_ny;
-    const int kxq = (int)(q % a.ptab_nx);
-    q /= a.ptab_nx;
+    // the faster of the two indices first (a.ptab_sx, a.ptab_sy)
+    const int nf = a.ptab_sy == 1 ? a.ptab_ny : a.ptab_nx, ns = a.ptab_sy == 1 ? a.ptab_nx : a.ptab_ny;
+    const int kf = (int)(i % nf);
+    long long q = i / nf;
+    const int ks = (int)(q % ns);
+    q /= ns;
+    const int kxq = a.ptab_sy == 1 ? ks : kf, kyq = a.ptab_sy == 1 ? kf : ks;
     const int iw = (int)(q % a.d.nw);
     const int r = (int)(q / a.d.nw);
     dst[i] = qmult<Q_PS_FWD>(b, r, iw, kxq, kyq);
