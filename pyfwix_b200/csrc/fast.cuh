@@ -23,6 +23,7 @@
 #include <cstring>
 #include <map>
 #include <tuple>
+#include <type_traits>
 #include <mutex>
 #include <utility>
 
@@ -96,7 +97,6 @@ struct Plan {
 };
 
 constexpr int kWarps = 8;       // warps per CTA in every pass
-constexpr int kMaxHatRefs = 32;  // smooth-step references the row passes stage in shared memory
 
 template <class P, bool REV>
 struct Order {
@@ -295,63 +295,15 @@ struct RowGeo {
   // shared-memory stride between lines
   static constexpr int LINE = P::N + (P::LINE_EXTRA > (P::T < 32 ? 8 : 0) ? P::LINE_EXTRA : (P::T < 32 ? 8 : 0));
   static constexpr int ROWS = kWarps * P::G;                // rows per CTA
-  // after the twiddles: the smooth step's references and inverse spans (kMaxHatRefs each)
-  static size_t smem() { return ((size_t)kWarps * P::G * LINE + tw_size<P>() + kMaxHatRefs) * sizeof(float2); }
+  static size_t smem() { return ((size_t)kWarps * P::G * LINE + tw_size<P>()) * sizeof(float2); }
   // Born-weight rows of the CTA staged after the above (16-byte aligned): nterm
   // tables x ROWS rows x N samples, when they fit in 160 KB
   __host__ __device__ static constexpr size_t scat_offset() {
-    return ((size_t)kWarps * P::G * LINE + tw_size<P>() + kMaxHatRefs + 1) & ~(size_t)1;
+    return ((size_t)kWarps * P::G * LINE + tw_size<P>() + 1) & ~(size_t)1;
   }
   __host__ __device__ static bool scat_stage(int nterm) { return (size_t)nterm * ROWS * P::N * 8 <= 160 * 1024; }
   static size_t smem_scat(int nterm) { return (scat_offset() + (size_t)nterm * ROWS * P::N) * sizeof(float2); }
 };
-
-// Smooth-step references of the row passes, staged in shared memory once per CTA:
-// ref[0 .. n) and inv[j] = 1 / (ref[j+1] - ref[j]).  With more references than
-// kMaxHatRefs the passes fall back to the per-term weights of row_weight.
-template <class P>
-__device__ __forceinline__ void stage_hat_refs(const SpecArgs& a, float* ref, float* inv) {
-  const int n = a.sm_n;
-  if ((int)threadIdx.x < n) {
-    const int i = threadIdx.x;
-    ref[i] = a.sm_ref[i];
-    inv[i] = i + 1 < n ? 1.f / (a.sm_ref[i + 1] - a.sm_ref[i]) : 0.f;
-  }
-}
-// Fractional reference index g of slowness s: the hat weights are 1 - (g - j) on
-// reference j and g - j on j + 1, j = min(floor g, n - 2); g = 0 and g = n - 1 are
-// the clamped ends (weight 1 on the end reference, derivative 0).  Same
-// bracketing as hat_weight.
-__device__ __forceinline__ float hat_index(const float* ref, const float* inv, int n, float s) {
-  if (n == 1 || s <= ref[0]) return 0.f;
-  if (s >= ref[n - 1]) return (float)(n - 1);
-  int j = 0;
-  while (j < n - 2 && s >= ref[j + 1]) ++j;
-  return (float)j + (s - ref[j]) * inv[j];
-}
-__device__ __forceinline__ unsigned hat_index_support(int n, float g) {
-  if (n == 1 || g <= 0.f) return 1u;
-  if (g >= (float)(n - 1)) return 1u << (n - 1);
-  return 3u << min((int)g, n - 2);
-}
-// Hat weight (x) and its slowness derivative (y) of reference t at index g.
-__device__ __forceinline__ float2 hat_at(const float* inv, int n, int t, float g) {
-  if (n == 1 || g <= 0.f) return make_float2(t == 0 ? 1.f : 0.f, 0.f);
-  if (g >= (float)(n - 1)) return make_float2(t == n - 1 ? 1.f : 0.f, 0.f);
-  const int j = min((int)g, n - 2);
-  const float u = g - (float)j;
-  if (t == j) return make_float2(1.f - u, -inv[j]);
-  if (t == j + 1) return make_float2(u, inv[j]);
-  return make_float2(0.f, 0.f);
-}
-// Reference part of the smooth weight from the hat: w C (W_SMOOTH), w conj(C)
-// (W_SMOOTH_CONJ), (w' - i w dz w) C (W_SMOOTH_DERIV).
-template <int W>
-__device__ __forceinline__ float2 hat_ref_weight(float2 h, float wdz, float2 C) {
-  if (W == W_SMOOTH) return cscale(C, h.x);
-  if (W == W_SMOOTH_CONJ) return cscale(cconj(C), h.x);
-  return cmul(make_float2(h.y, -wdz * h.x), C);
-}
 
 // Per-thread view of a row pass: which row, which lane of the line, its smem line.
 template <class P>
@@ -430,9 +382,13 @@ __global__ void __launch_bounds__(kWarps * 32, row_fwd_min_blocks<P, PRE>()) k_r
     cp_async_commit();
   }
   load_stage_tw<P>(c.tw, a.twx);
-  if (PRE == W_SMOOTH_CONJ && a.sm_n <= kMaxHatRefs)
-    stage_hat_refs<P>(a, reinterpret_cast<float*>(c.tw + tw_size<P>()),
-                      reinterpret_cast<float*>(c.tw + tw_size<P>()) + kMaxHatRefs);
+  constexpr bool kSmooth = PRE == W_SMOOTH_CONJ;
+  __shared__ typename std::conditional<kSmooth, HatTables, int>::type hat;
+  float unit = 0.f;
+  if constexpr (kSmooth) {
+    unit = phase_unit(a, c.iw);
+    stage_hat(hat, a, c.iw, unit);
+  }
   __syncthreads();
   float2 raw[P::E];
   const long long roff = (c.b * a.d.NY + (c.live ? c.y : 0)) * P::N;
@@ -474,30 +430,24 @@ __global__ void __launch_bounds__(kWarps * 32, row_fwd_min_blocks<P, PRE>()) k_r
 #pragma unroll
     for (int e = 0; e < P::E; ++e) lab.set(e, c.live ? lrow[pos_first<P>(c.t, e)] : 255u);
   }
-  // smooth weights (references staged in shared memory): each cell's fractional
-  // reference index and the cell part conj(B(s)) of every reference's weight,
-  // once per cell; terms that no sample of the warp's rows supports are zero rows
-  constexpr bool kSmooth = PRE == W_SMOOTH_CONJ;
+  // smooth weights: each cell's fractional reference index and the cell part
+  // conj(B(s)) of every reference's weight, once per cell; terms that no sample of
+  // the warp's rows supports are zero rows
   unsigned used = 0xffffffffu;
   float g[kSmooth ? P::E : 1];
-  const float* href = reinterpret_cast<const float*>(c.tw + tw_size<P>());
-  const float* hinv = href + kMaxHatRefs;
-  const bool hat_smem = kSmooth && a.sm_n <= kMaxHatRefs;
-  if (hat_smem) {
+  if constexpr (kSmooth) {
     const float* srow = a.sm_s + (long long)(c.live ? c.y : 0) * P::N;
     unsigned mine = 0;
 #pragma unroll
     for (int e = 0; e < P::E; ++e) {
       const float sv = c.live ? srow[pos_first<P>(c.t, e)] : 0.f;
-      g[e] = hat_index(href, hinv, a.sm_n, sv);
+      g[e] = hat_index(hat, a.sm_n, sv);
       if (c.live) {
         mine |= hat_index_support(a.sm_n, g[e]);
-        raw[e] = cmul_conj(raw[e], smooth_cell_phase(a, c.iw, sv));
+        raw[e] = cmul_conj(raw[e], smooth_cell_phase(unit, sv));
       }
     }
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) mine |= __shfl_xor_sync(0xffffffffu, mine, o);
-    used = mine;
+    used = __reduce_or_sync(0xffffffffu, mine);
   }
   if (scat_smem) {  // the weight rows have landed (the input rows are in registers)
     cp_async_wait<0>();
@@ -513,13 +463,10 @@ __global__ void __launch_bounds__(kWarps * 32, row_fwd_min_blocks<P, PRE>()) k_r
       }
       continue;
     }
-    if (hat_smem) {
-      const float2 C = smooth_ref_phase(a, c.iw, term);
-      const float wdz = a.w[c.iw] * a.dz;
+    if constexpr (kSmooth) {
+      const float2 C = hat.C[term];
 #pragma unroll
-      for (int e = 0; e < P::E; ++e)
-        v[e] = c.live ? cmul(raw[e], hat_ref_weight<PRE>(hat_at(hinv, a.sm_n, term, g[e]), wdz, C))
-                      : make_float2(0.f, 0.f);
+      for (int e = 0; e < P::E; ++e) v[e] = cmul_conj(cscale(raw[e], hat_w(g[e], term)), C);  // raw is 0 where !live
     } else if (kScatC && scat_smem) {
       const float f = 0.5f * a.w[c.iw] * a.dz * a.coef[term + a.term0];
       const float2* wrow = wt + ((size_t)term * RowGeo<P>::ROWS + (c.y - y0)) * P::N;
@@ -590,19 +537,22 @@ __global__ void __launch_bounds__(kWarps * 32, multi_term(POST) && (P::E == 16 |
   }
   bool wt_ready = false;
   load_stage_tw<P>(c.tw, a.twx);
-  constexpr bool kPair = POST == W_SMOOTH_PAIR;
-  constexpr bool kSmooth = POST == W_SMOOTH || POST == W_SMOOTH_DERIV || kPair;
-  const bool hat_smem = kSmooth && a.sm_n <= kMaxHatRefs;
-  const float* href = reinterpret_cast<const float*>(c.tw + tw_size<P>());
-  const float* hinv = href + kMaxHatRefs;
-  if (hat_smem) stage_hat_refs<P>(a, const_cast<float*>(href), const_cast<float*>(hinv));
+  // kDeriv: the sum of w_r' C_r T_r beside the step's own
+  constexpr bool kPair = POST == W_SMOOTH_PAIR, kDeriv = kPair || POST == W_SMOOTH_DERIV;
+  constexpr bool kSmooth = POST == W_SMOOTH || kDeriv;
+  __shared__ typename std::conditional<kSmooth, HatTables, int>::type hat;
+  float unit = 0.f;
+  if constexpr (kSmooth) {
+    unit = phase_unit(a, c.iw);
+    stage_hat(hat, a, c.iw, unit);
+  }
   __syncthreads();
   float g[kSmooth ? P::E : 1];
   float2 acc[P::E];
-  float2 acc2[kPair ? P::E : 1];
+  float2 acc2[kDeriv ? P::E : 1];
 #pragma unroll
   for (int e = 0; e < P::E; ++e) acc[e] = make_float2(0.f, 0.f);
-  if constexpr (kPair) {
+  if constexpr (kDeriv) {
 #pragma unroll
     for (int e = 0; e < P::E; ++e) acc2[e] = make_float2(0.f, 0.f);
   }
@@ -621,17 +571,16 @@ __global__ void __launch_bounds__(kWarps * 32, multi_term(POST) && (P::E == 16 |
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) mine |= __shfl_xor_sync(0xffffffffu, mine, o);
     used = nterm > 32 ? 0xffffffffu : mine;
-  } else if (hat_smem) {
+  }
+  if constexpr (kSmooth) {
     unsigned mine = 0;
     const float* srow = a.sm_s + (long long)(c.live ? c.y : 0) * P::N;
 #pragma unroll
     for (int e = 0; e < P::E; ++e) {
-      g[e] = hat_index(href, hinv, a.sm_n, c.live ? srow[pos_first<P>(c.t, e)] : 0.f);
+      g[e] = hat_index(hat, a.sm_n, c.live ? srow[pos_first<P>(c.t, e)] : 0.f);
       if (c.live) mine |= hat_index_support(a.sm_n, g[e]);
     }
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) mine |= __shfl_xor_sync(0xffffffffu, mine, o);
-    used = mine;
+    used = __reduce_or_sync(0xffffffffu, mine);
   }
   auto next_term = [&](int from) {
     int k = from;
@@ -642,7 +591,7 @@ __global__ void __launch_bounds__(kWarps * 32, multi_term(POST) && (P::E == 16 |
   int term = next_term(0);
   // the next term's row is prefetched, except where the paired sums of 16-sample
   // lanes leave no registers for it (two accumulators, the term and the hat indices)
-  constexpr bool kPrefetch = FWIX_ROWINV_PREFETCH && !(kPair && P::E >= 16);
+  constexpr bool kPrefetch = FWIX_ROWINV_PREFETCH && !(kDeriv && P::E >= 16);
   float2 pre[kPrefetch ? P::E : 1];
   if (kPrefetch && term < nterm) {
     const float2* src = a.t2 + (long long)term * a.tstride + roff;
@@ -666,20 +615,15 @@ __global__ void __launch_bounds__(kWarps * 32, multi_term(POST) && (P::E == 16 |
       for (int e = 0; e < P::E; ++e) pre[e] = c.live ? src[pos_last<P>(c.t, e)] : make_float2(0.f, 0.f);
     }
     fft_inv<P>(v, c.t, c.tw, c.line);
-    if (hat_smem) {
+    if constexpr (kSmooth) {
       // reference part of the weights here, the cell part B(s) once after the sum
-      const float2 C = smooth_ref_phase(a, c.iw, term);
-      const float wdz = a.w[c.iw] * a.dz;
+      const float2 C = hat.C[term];
+      const float below = hat.inv[term > 0 ? term - 1 : 0], above = hat.inv[term];
 #pragma unroll
       for (int e = 0; e < P::E; ++e) {
-        if (!c.live) continue;
-        const float2 h = hat_at(hinv, a.sm_n, term, g[e]);
-        if constexpr (kPair) {
-          acc[e] = cadd(acc[e], cmul(v[e], hat_ref_weight<W_SMOOTH>(h, wdz, C)));
-          acc2[e] = cadd(acc2[e], cmul(v[e], hat_ref_weight<W_SMOOTH_DERIV>(h, wdz, C)));
-        } else {
-          acc[e] = cadd(acc[e], cmul(v[e], hat_ref_weight<POST>(h, wdz, C)));
-        }
+        const float2 u = cmul(v[e], C);
+        acc[e] = cfma(u, hat_w(g[e], term), acc[e]);
+        if constexpr (kDeriv) acc2[e] = cfma(u, hat_dw(g[e], term, a.sm_n, below, above), acc2[e]);
       }
     } else if (kScat && scat_smem) {
       if (!wt_ready) {  // every warp reaches this after its first transform (no term is skipped)
@@ -698,12 +642,7 @@ __global__ void __launch_bounds__(kWarps * 32, multi_term(POST) && (P::E == 16 |
         if (POST == W_MASK) {
           if (lab.get(e) == term) acc[e] = v[e];
         } else if (c.live) {
-          if constexpr (kPair) {
-            acc[e] = cadd(acc[e], row_weight<W_SMOOTH>(a, term, c.iw, c.y, pos_first<P>(c.t, e), v[e]));
-            acc2[e] = cadd(acc2[e], row_weight<W_SMOOTH_DERIV>(a, term, c.iw, c.y, pos_first<P>(c.t, e), v[e]));
-          } else {
-            acc[e] = cadd(acc[e], row_weight<POST>(a, term, c.iw, c.y, pos_first<P>(c.t, e), v[e]));
-          }
+          acc[e] = cadd(acc[e], row_weight<POST>(a, term, c.iw, c.y, pos_first<P>(c.t, e), v[e]));
         }
       }
     }
@@ -714,14 +653,16 @@ __global__ void __launch_bounds__(kWarps * 32, multi_term(POST) && (P::E == 16 |
   float2* dst2 = kPair ? a.out2 + (c.b * a.d.NY + c.y) * P::N : nullptr;
   const float ty = post_taper ? a.tapy[c.y] : 1.f;
   const float* srow_out = kSmooth ? a.sm_s + (long long)c.y * P::N : nullptr;
+  const float wdz = a.w[c.iw] * a.dz;
 #pragma unroll
   for (int e = 0; e < P::E; ++e) {
     const int x = pos_first<P>(c.t, e);
     float2 v = acc[e];
     float2 cell = make_float2(1.f, 0.f);
-    if (hat_smem) {
-      cell = smooth_cell_phase(a, c.iw, srow_out[x]);
-      v = cmul(v, cell);
+    if constexpr (kSmooth) {
+      cell = smooth_cell_phase(unit, srow_out[x]);
+      if constexpr (kDeriv) acc2[e] = cfma(rot90<false>(v), wdz, acc2[e]);  // S1 - i w dz S
+      v = cmul(POST == W_SMOOTH_DERIV ? acc2[kDeriv ? e : 0] : v, cell);
     }
     if constexpr (POST == W_ONE_DIRECT) v = cadd(v, scat_direct(a, c.b, c.iw, c.y, x));
     if (post_taper) v = cscale(v, a.tapx[x] * ty);
@@ -738,7 +679,7 @@ __global__ void __launch_bounds__(kWarps * 32, multi_term(POST) && (P::E == 16 |
       atomicAdd(a.ic_img + (long long)c.y * a.d.nx + x, bg.x * v.x + bg.y * v.y);
     }
     if constexpr (kPair) {
-      float2 u = hat_smem ? cmul(acc2[e], cell) : acc2[e];
+      float2 u = cmul(acc2[e], cell);
       if (post_taper) u = cscale(u, a.tapx[x] * ty);
       if (a.add) u = cadd(dst2[x], u);
       dst2[x] = u;

@@ -125,9 +125,9 @@ struct Dim {
 // threads per SM, by the largest radix (a radix's samples are 2 registers each,
 // and a pass holds two to three such sets).
 template <class S>
-constexpr int min_blocks(int threads, bool light = false) {
+constexpr int min_blocks(int threads, bool light = false, bool heavy = false) {
   if (!S::kFixed) return 1;
-  const int want = light ? 1024 : S::MAXR <= 10 ? 768 : S::MAXR <= 16 ? 640 : 512;
+  const int want = light ? 1024 : heavy ? 512 : S::MAXR <= 10 ? 768 : S::MAXR <= 16 ? 640 : 512;
   return want / threads < 1 ? 1 : want / threads;
 }
 
@@ -288,24 +288,7 @@ struct RowCtx {
 
 // Classes of row weights that share a kernel (the weight itself is a uniform
 // run-time switch within a class).
-enum RowClass { C_ONE, C_MASK, C_SCAT, C_SMOOTH, C_PAIR };
-inline int row_class(int w) {
-  switch (w) {
-    case W_MASK: return C_MASK;
-    case W_SCAT:
-    case W_SCAT_CONJ: return C_SCAT;
-    case W_SMOOTH:
-    case W_SMOOTH_CONJ:
-    case W_SMOOTH_DERIV: return C_SMOOTH;
-    case W_SMOOTH_PAIR: return C_PAIR;
-    default: return C_ONE;
-  }
-}
-
-// Terms a cell's smooth weight can be nonzero for (all beyond 32 references).
-__device__ __forceinline__ unsigned smooth_support(const SpecArgs& a, float s) {
-  return a.sm_n <= 32 ? hat_support(a.sm_ref, a.sm_n, s) : 0xffffffffu;
-}
+enum RowClass { C_ONE, C_MASK, C_SCAT, C_SMOOTH, C_PAIR, C_DERIV };
 
 // t1[term] = F_x(pre_term * in) for each term.  The row's samples are read once
 // into registers; a term whose weight vanishes on all of the CTA's rows (masks,
@@ -321,6 +304,13 @@ __global__ void __launch_bounds__(S::ROW_THREADS, min_blocks<S>(S::ROW_THREADS, 
   float2* const buf1 = buf0 + d.rows() * row_ls(d.n(), S::RT);
   const RowCtx<S> c(a, d);
   const RowPlace<S, false> w(d);
+  constexpr bool kSmooth = CLS == C_SMOOTH;
+  __shared__ typename std::conditional<kSmooth, HatTables, int>::type hat;
+  float unit = 0.f;
+  if constexpr (kSmooth) {
+    unit = phase_unit(a, c.iw);
+    stage_hat(hat, a, c.iw, unit);
+  }
   fill_twiddles(tw, a.twx, RT, d.rb(), d.ra(), d.row_threads());
   const long long roff = (c.b * a.d.NY + (c.live ? c.y : 0)) * d.n();
   float2 raw[RT];
@@ -359,16 +349,25 @@ __global__ void __launch_bounds__(S::ROW_THREADS, min_blocks<S>(S::ROW_THREADS, 
       if (lab[r] < 32) mine |= 1u << lab[r];
     }
     used = a.nterm > 32 ? 0xffffffffu : cta_or(mine);
-  } else if (CLS == C_SMOOTH) {
-    unsigned mine = 0;
-    if (c.live) {
-      const float* srow = a.sm_s + (long long)c.y * d.n();
-#pragma unroll
-      for (int r = 0; r < RT; ++r) mine |= smooth_support(a, srow[c.j + r * d.nt()]);
-    }
-    used = cta_or(mine);
   } else {
     __syncthreads();
+  }
+  // smooth weights: a cell's fractional reference index, and the cell part conj(B(s))
+  // of every reference's weight once per cell
+  float hg[kSmooth ? RT : 1];
+  if constexpr (kSmooth) {
+    unsigned mine = 0;
+    const float* srow = a.sm_s + (long long)(c.live ? c.y : 0) * d.n();
+#pragma unroll
+    for (int r = 0; r < RT; ++r) {
+      const float sv = c.live ? srow[c.j + r * d.nt()] : 0.f;
+      hg[r] = hat_index(hat, a.sm_n, sv);
+      if (c.live) {
+        mine |= hat_index_support(a.sm_n, hg[r]);
+        raw[r] = cmul_conj(raw[r], smooth_cell_phase(unit, sv));
+      }
+    }
+    used = cta_or(mine);
   }
   const int nterm = CLS == C_ONE ? 1 : a.nterm;
   int k = 0;  // terms transformed so far
@@ -390,10 +389,10 @@ __global__ void __launch_bounds__(S::ROW_THREADS, min_blocks<S>(S::ROW_THREADS, 
 #pragma unroll
         for (int r = 0; r < RT; ++r)
           v[r] = c.live ? row_weight<W_SCAT_CONJ>(a, term, c.iw, c.y, c.j + r * d.nt(), raw[r]) : raw[r];
-      } else if (CLS == C_SMOOTH) {
+      } else if constexpr (kSmooth) {
+        const float2 C = hat.C[term];
 #pragma unroll
-        for (int r = 0; r < RT; ++r)
-          v[r] = c.live ? row_weight<W_SMOOTH_CONJ>(a, term, c.iw, c.y, c.j + r * d.nt(), raw[r]) : raw[r];
+        for (int r = 0; r < RT; ++r) v[r] = cmul_conj(cscale(raw[r], hat_w(hg[r], term)), C);
       } else {
 #pragma unroll
         for (int r = 0; r < RT; ++r) v[r] = raw[r];
@@ -430,7 +429,7 @@ __global__ void __launch_bounds__(S::ROW_THREADS, min_blocks<S>(S::ROW_THREADS, 
 // out (+)= post * sum_term W_term * F_x^-1(t2[term]); terms that no sample of the
 // CTA's rows selects are skipped.
 template <class S, int CLS>
-__global__ void __launch_bounds__(S::ROW_THREADS, min_blocks<S>(S::ROW_THREADS, CLS == C_ONE))
+__global__ void __launch_bounds__(S::ROW_THREADS, min_blocks<S>(S::ROW_THREADS, CLS == C_ONE, CLS == C_PAIR || CLS == C_DERIV))
     k_row_inv(const SpecArgs a, const __grid_constant__ Geo g, int post, int post_taper) {
   constexpr int RT = S::RT;
   const Dim<S> d{g};
@@ -440,14 +439,22 @@ __global__ void __launch_bounds__(S::ROW_THREADS, min_blocks<S>(S::ROW_THREADS, 
   float2* const buf1 = buf0 + d.rows() * row_ls(d.n(), d.ra());
   const RowCtx<S> c(a, d);
   const RowPlace<S, true> w(d);
+  // kDeriv: the sum of w_r' C_r T_r beside the step's own
+  constexpr bool kDeriv = CLS == C_PAIR || CLS == C_DERIV, kSmooth = CLS == C_SMOOTH || kDeriv;
+  __shared__ typename std::conditional<kSmooth, HatTables, int>::type hat;
+  float unit = 0.f;
+  if constexpr (kSmooth) {
+    unit = phase_unit(a, c.iw);
+    stage_hat(hat, a, c.iw, unit);
+  }
   fill_twiddles(tw, a.twx, d.ra(), d.rb(), RT, d.row_threads());
   float2 acc[RT];
-  float2 acc2[CLS == C_PAIR ? RT : 1];
+  float2 acc2[kDeriv ? RT : 1];
 #pragma unroll
   for (int r = 0; r < RT; ++r) acc[r] = make_float2(0.f, 0.f);
-  if (CLS == C_PAIR) {
+  if constexpr (kDeriv) {
 #pragma unroll
-    for (int r = 0; r < RT; ++r) acc2[CLS == C_PAIR ? r : 0] = make_float2(0.f, 0.f);
+    for (int r = 0; r < RT; ++r) acc2[r] = make_float2(0.f, 0.f);
   }
   int lab[CLS == C_MASK ? RT : 1];
   unsigned used = 0xffffffffu;
@@ -460,16 +467,19 @@ __global__ void __launch_bounds__(S::ROW_THREADS, min_blocks<S>(S::ROW_THREADS, 
       if (lab[r] < 32) mine |= 1u << lab[r];
     }
     used = a.nterm > 32 ? 0xffffffffu : cta_or(mine);
-  } else if (CLS == C_SMOOTH || CLS == C_PAIR) {
-    unsigned mine = 0;
-    if (c.live) {
-      const float* srow = a.sm_s + (long long)c.y * d.n();
-#pragma unroll
-      for (int r = 0; r < RT; ++r) mine |= smooth_support(a, srow[c.j + r * d.nt()]);
-    }
-    used = cta_or(mine);
   } else {
     __syncthreads();
+  }
+  float hg[kSmooth ? RT : 1];
+  if constexpr (kSmooth) {
+    unsigned mine = 0;
+    const float* srow = a.sm_s + (long long)(c.live ? c.y : 0) * d.n();
+#pragma unroll
+    for (int r = 0; r < RT; ++r) {
+      hg[r] = hat_index(hat, a.sm_n, c.live ? srow[c.j + r * d.nt()] : 0.f);
+      if (c.live) mine |= hat_index_support(a.sm_n, hg[r]);
+    }
+    used = cta_or(mine);
   }
   const int nterm = CLS == C_ONE ? 1 : a.nterm;
   int k = 0;
@@ -513,22 +523,15 @@ __global__ void __launch_bounds__(S::ROW_THREADS, min_blocks<S>(S::ROW_THREADS, 
 #pragma unroll
       for (int r = 0; r < RT; ++r)
         acc[r] = cadd(acc[r], row_weight<W_SCAT>(a, term, c.iw, c.y, c.j + r * d.nt(), v[r]));
-    } else if (CLS == C_SMOOTH) {
-      if (post == W_SMOOTH) {
-#pragma unroll
-        for (int r = 0; r < RT; ++r)
-          acc[r] = cadd(acc[r], row_weight<W_SMOOTH>(a, term, c.iw, c.y, c.j + r * d.nt(), v[r]));
-      } else {
-#pragma unroll
-        for (int r = 0; r < RT; ++r)
-          acc[r] = cadd(acc[r], row_weight<W_SMOOTH_DERIV>(a, term, c.iw, c.y, c.j + r * d.nt(), v[r]));
-      }
-    } else if (CLS == C_PAIR) {
+    } else if constexpr (kSmooth) {
+      // reference part of the weights here, the cell part B(s) once after the sum
+      const float2 C = hat.C[term];
+      const float below = hat.inv[term > 0 ? term - 1 : 0], above = hat.inv[term];
 #pragma unroll
       for (int r = 0; r < RT; ++r) {
-        const int x = c.j + r * d.nt(), q = CLS == C_PAIR ? r : 0;
-        acc[r] = cadd(acc[r], row_weight<W_SMOOTH>(a, term, c.iw, c.y, x, v[r]));
-        acc2[q] = cadd(acc2[q], row_weight<W_SMOOTH_DERIV>(a, term, c.iw, c.y, x, v[r]));
+        const float2 u = cmul(v[r], C);
+        acc[r] = cfma(u, hat_w(hg[r], term), acc[r]);
+        if constexpr (kDeriv) acc2[r] = cfma(u, hat_dw(hg[r], term, a.sm_n, below, above), acc2[r]);
       }
     } else {
 #pragma unroll
@@ -538,10 +541,17 @@ __global__ void __launch_bounds__(S::ROW_THREADS, min_blocks<S>(S::ROW_THREADS, 
   if (!c.live) return;
   const long long roff = (c.b * a.d.NY + c.y) * d.n();
   const float ty = post_taper ? a.tapy[c.y] : 1.f;
+  const float wdz = a.w[c.iw] * a.dz;
 #pragma unroll
   for (int r = 0; r < RT; ++r) {
     const int x = c.j + r * d.nt();
     float2 v = acc[r];
+    float2 cell = make_float2(1.f, 0.f);
+    if constexpr (kSmooth) {
+      cell = smooth_cell_phase(unit, a.sm_s[(long long)c.y * d.n() + x]);
+      if constexpr (kDeriv) acc2[r] = cfma(rot90<false>(v), wdz, acc2[r]);  // S1 - i w dz S
+      v = cmul(CLS == C_DERIV ? acc2[kDeriv ? r : 0] : v, cell);
+    }
     if (CLS == C_ONE && post == W_ONE_DIRECT) v = cadd(v, scat_direct(a, c.b, c.iw, c.y, x));
     if (post_taper) v = cscale(v, a.tapx[x] * ty);
     if (a.add) v = cadd(a.out[roff + x], v);
@@ -553,7 +563,7 @@ __global__ void __launch_bounds__(S::ROW_THREADS, min_blocks<S>(S::ROW_THREADS, 
       atomicAdd(a.ic_img + (long long)c.y * a.d.nx + x, bg.x * v.x + bg.y * v.y);
     }
     if (CLS == C_PAIR) {
-      float2 u = acc2[CLS == C_PAIR ? r : 0];
+      float2 u = cmul(acc2[kDeriv ? r : 0], cell);
       if (post_taper) u = cscale(u, a.tapx[x] * ty);
       if (a.add) u = cadd(a.out2[roff + x], u);
       a.out2[roff + x] = u;
@@ -947,8 +957,8 @@ cudaError_t row_inverse_s(const SpecArgs& a, const Line& p, int post, int pt, cu
     case W_ONE_DIRECT: return launch(k_row_inv<S, C_ONE>, grid, th, sm, s, a, g, post, pt);
     case W_MASK: return launch(k_row_inv<S, C_MASK>, grid, th, sm, s, a, g, post, pt);
     case W_SCAT: return launch(k_row_inv<S, C_SCAT>, grid, th, sm, s, a, g, post, pt);
-    case W_SMOOTH:
-    case W_SMOOTH_DERIV: return launch(k_row_inv<S, C_SMOOTH>, grid, th, sm, s, a, g, post, pt);
+    case W_SMOOTH: return launch(k_row_inv<S, C_SMOOTH>, grid, th, sm, s, a, g, post, pt);
+    case W_SMOOTH_DERIV: return launch(k_row_inv<S, C_DERIV>, grid, th, sm, s, a, g, post, pt);
     case W_SMOOTH_PAIR: return launch(k_row_inv<S, C_PAIR>, grid, th, sm, s, a, g, post, pt);
     default: return cudaErrorInvalidValue;
   }

@@ -96,28 +96,67 @@ __device__ __forceinline__ unsigned hat_support(const float* ref, int n, float s
 
 // The split-step factor of the smooth step factors into a cell part and a
 // reference part: SS_r = exp(-i w (s - s_r) dz) = B(s) C_r with B(s) =
-// exp(-i w s dz) and C_r = exp(i w s_r dz).  The register-resident row passes use
-// it to take one sine / cosine per cell (B, applied once to the sum over
-// references, or once to the input of the adjoint) and one per reference and
-// line (C_r) instead of one per cell and reference.
-__device__ __forceinline__ float2 smooth_cell_phase(const SpecArgs& a, int iw, float s) {  // B(s)
+// exp(-i w s dz) and C_r = exp(i w s_r dz).  The register-resident row passes
+// take one sine / cosine per cell (B, applied once to the sum over references, or
+// once to the input of the adjoint) and one per reference and CTA (C_r, in shared
+// memory).  The hat weight of reference t is max(0, 1 - |g - t|) at a cell's
+// fractional reference index g, a real factor of t's transform, and the
+// derivative (w_r' - i w dz w_r) SS_r needs only the sum S1 of w_r' C_r T_r beside
+// the step's own sum S of w_r C_r T_r: it is (S1 - i w dz S) B.  (With a complex
+// weight per cell and term, sines of C_r in every lane and branches for the hat the
+// 384 x 384 x 96 inverse row passes took 373 us (step), 395 (derivative) and 476
+// (both) and the forward one 323; now 293, 312, 324 and 249.)
+constexpr int kMaxRefs = 256;  // more than a plan can have
+struct HatTables {
+  float ref[kMaxRefs];
+  float inv[kMaxRefs];  // 1 / (ref[j+1] - ref[j])
+  float2 C[kMaxRefs];
+};
+// w dz / pi of frequency iw: phases go to sincospif, whose range reduction is exact.
+__device__ __forceinline__ float phase_unit(const SpecArgs& a, int iw) {
+  return (float)((double)a.w[iw] * (double)a.dz * 0.31830988618379067154);
+}
+// Tables of the CTA's frequency iw (a barrier must follow).
+__device__ __forceinline__ void stage_hat(HatTables& h, const SpecArgs& a, int iw, float unit) {
+  for (int i = threadIdx.x; i < a.sm_n; i += blockDim.x) {
+    const float s = a.sm_ref[i];
+    float sn, cs;
+    sincospif(unit * s, &sn, &cs);
+    h.ref[i] = s;
+    h.inv[i] = i + 1 < a.sm_n ? 1.f / (a.sm_ref[i + 1] - s) : 0.f;
+    h.C[i] = make_float2(cs, sn);
+  }
+}
+__device__ __forceinline__ float2 smooth_cell_phase(float unit, float s) {  // B(s)
   float sn, cs;
-  sincosf(a.w[iw] * a.dz * s, &sn, &cs);
+  sincospif(unit * s, &sn, &cs);
   return make_float2(cs, -sn);
 }
-__device__ __forceinline__ float2 smooth_ref_phase(const SpecArgs& a, int iw, int t) {  // C_t
-  float sn, cs;
-  sincosf(a.w[iw] * a.dz * a.sm_ref[t], &sn, &cs);
-  return make_float2(cs, sn);
+// Fractional reference index g of slowness s: the hat weights are 1 - (g - j) on
+// reference j and g - j on j + 1, j = min(floor g, n - 2); g = 0 and g = n - 1 are
+// the clamped ends (weight 1 on the end reference, derivative 0).  Same
+// bracketing as hat_weight.
+__device__ __forceinline__ float hat_index(const HatTables& h, int n, float s) {
+  if (n == 1 || s <= h.ref[0]) return 0.f;
+  if (s >= h.ref[n - 1]) return (float)(n - 1);
+  int j = 0;
+  for (int k = 1; k < n - 1; ++k) j += s >= h.ref[k] ? 1 : 0;
+  return (float)j + (s - h.ref[j]) * h.inv[j];
 }
-// Reference part of the weight of term t at slowness s: w_t C_t (W_SMOOTH),
-// w_t conj(C_t) (W_SMOOTH_CONJ) or (w_t' - i w dz w_t) C_t (W_SMOOTH_DERIV).
-template <int W>
-__device__ __forceinline__ float2 smooth_ref_weight(const SpecArgs& a, int t, int iw, float s, float2 C) {
-  const Hat h = hat_weight(a.sm_ref, a.sm_n, t, s);
-  if (W == W_SMOOTH) return cscale(C, h.w);
-  if (W == W_SMOOTH_CONJ) return cscale(cconj(C), h.w);
-  return cmul(make_float2(h.dw, -a.w[iw] * a.dz * h.w), C);
+// Terms that index g gives a weight or derivative (n <= 32; every bit beyond).
+__device__ __forceinline__ unsigned hat_index_support(int n, float g) {
+  if (n > 32) return 0xffffffffu;
+  if (n == 1 || g <= 0.f) return 1u;
+  if (g >= (float)(n - 1)) return 1u << (n - 1);
+  return 3u << min((int)g, n - 2);
+}
+__device__ __forceinline__ float hat_w(float g, int t) { return __saturatef(1.f - fabsf(g - (float)t)); }
+// Slowness derivative of reference t's weight (interval j = floor g: -inv[j] on j,
+// inv[j] on j + 1).
+__device__ __forceinline__ float hat_dw(float g, int t, int n, float inv_below, float inv_above) {
+  const float d = g - (float)t;
+  const float v = d >= 0.f ? (d < 1.f ? -inv_above : 0.f) : (d >= -1.f ? inv_below : 0.f);
+  return g > 0.f && g < (float)(n - 1) ? v : 0.f;
 }
 
 // w_r SS_r (W_SMOOTH), w_r conj(SS_r) (W_SMOOTH_CONJ) or (w_r' - i w dz w_r) SS_r
