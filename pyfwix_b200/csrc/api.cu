@@ -347,6 +347,7 @@ fwix_status do_step(fwix_plan* p, int kind, int iz, int dir, const float2* in, f
   // intermediates; one chunk's column pass overlaps the next chunk's row pass.
   FWIX_CU(cudaEventRecord(p->lane_fork, s));
   FWIX_CU(cudaStreamWaitEvent(p->lane_s, p->lane_fork, 0));
+  a0.d.chained = 0;  // the lanes fill each other's tails
   const long long B = (long long)p->d.ns * p->d.nw;
   fwix_status st = FWIX_OK;
   int k = 0;
@@ -743,6 +744,7 @@ fwix_status fwix_plan_create(const fwix_desc* desc, fwix_plan** out) {
   p->d.ns = q.ns;
   p->d.slice = (long long)p->d.NX * p->d.NY;
   p->d.wfld = p->d.slice * q.nw * q.ns;
+  p->d.chained = 1;
   if (!make_fft_plan(p->d.NX, &p->px) || !make_fft_plan(p->d.NY, &p->py)) {
     delete p;
     return fail(FWIX_ERR_UNSUPPORTED, "wavefield sizes must be 2^a 3^b 5^c 7^d and at most 1024");
@@ -786,6 +788,9 @@ fwix_status fwix_plan_create(const fwix_desc* desc, fwix_plan** out) {
   if (e == cudaSuccess) e = cudaMalloc((void**)&p->rf_tab, (size_t)2 * p->d.nx * p->d.ny * sizeof(float2));
   if (e == cudaSuccess) e = cudaMalloc((void**)&p->err, sizeof(unsigned));
   if (e == cudaSuccess) e = cudaMemset(p->err, 0, sizeof(unsigned));
+  // the tables are on the device when the plan is handed out: chained passes
+  // read them before they wait for the stream (launch_chained)
+  if (e == cudaSuccess) e = cudaStreamSynchronize(0);
   if (e != cudaSuccess) {
     fwix_plan_destroy(p);
     return fail(FWIX_ERR_CUDA, std::string("plan tables: ") + cudaGetErrorString(e));
@@ -1670,8 +1675,14 @@ fwix_status fwix_sweep(int kind, const fwix_instance* insts, int ninst, void* co
     if (lanes[k].empty()) continue;
     cudaStream_t sk = (cudaStream_t)streams[k];
     e = cudaStreamWaitEvent(sk, fork, 0);
-    for (size_t j = 0; j < lanes[k].size() && e == cudaSuccess && st == FWIX_OK; ++j)
-      st = sweep_one(kind, insts[lanes[k][j]], sk);
+    for (size_t j = 0; j < lanes[k].size() && e == cudaSuccess && st == FWIX_OK; ++j) {
+      const fwix_instance& q = insts[lanes[k][j]];
+      // instances on several streams fill each other's tails: no early starts
+      const int chained = q.plan->d.chained;
+      if (std::min(ninst, nstreams) > 1) q.plan->d.chained = 0;
+      st = sweep_one(kind, q, sk);
+      q.plan->d.chained = chained;
+    }
     cudaEvent_t join = nullptr;
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&join, cudaEventDisableTiming);
     if (e == cudaSuccess) {

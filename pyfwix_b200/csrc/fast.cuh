@@ -361,6 +361,9 @@ template <class P, int PRE, bool RF = false>
 __global__ void __launch_bounds__(kWarps * 32, row_fwd_min_blocks<P, PRE>()) k_row_fwd(const SpecArgs a, int nchunk) {
   extern __shared__ float2 smem[];
   RowCtx<P> c(a, smem, nchunk);
+  chain_next();
+  load_stage_tw<P>(c.tw, a.twx);
+  chain_wait();
   prefetch_next_ctas<P::N, RowGeo<P>::ROWS>(a, a.in, false, nchunk);
   if constexpr (RF) prefetch_refl_rows<P>(a, c.b, (int)(blockIdx.x - c.bl * nchunk) * RowGeo<P>::ROWS, RowGeo<P>::ROWS);
   // Born weights (W_SCAT_CONJ) from the per-depth table: the CTA's rows of every
@@ -381,7 +384,6 @@ __global__ void __launch_bounds__(kWarps * 32, row_fwd_min_blocks<P, PRE>()) k_r
     }
     cp_async_commit();
   }
-  load_stage_tw<P>(c.tw, a.twx);
   constexpr bool kSmooth = PRE == W_SMOOTH_CONJ;
   __shared__ typename std::conditional<kSmooth, HatTables, int>::type hat;
   float unit = 0.f;
@@ -506,6 +508,9 @@ __global__ void __launch_bounds__(kWarps * 32, multi_term(POST) && (P::E == 16 |
     k_row_inv(const SpecArgs a, int nchunk, int post_taper) {
   extern __shared__ float2 smem[];
   RowCtx<P> c(a, smem, nchunk);
+  chain_next();
+  load_stage_tw<P>(c.tw, a.twx);
+  chain_wait();
   prefetch_next_ctas<P::N, RowGeo<P>::ROWS>(a, a.t2, true, nchunk);  // the first term of a later CTA
   // the reflection fields (the direct term's field) are read in the epilogue:
   // their rows head for L2 now
@@ -536,7 +541,6 @@ __global__ void __launch_bounds__(kWarps * 32, multi_term(POST) && (P::E == 16 |
     cp_async_commit();
   }
   bool wt_ready = false;
-  load_stage_tw<P>(c.tw, a.twx);
   // kDeriv: the sum of w_r' C_r T_r beside the step's own
   constexpr bool kPair = POST == W_SMOOTH_PAIR, kDeriv = kPair || POST == W_SMOOTH_DERIV;
   constexpr bool kSmooth = POST == W_SMOOTH || kDeriv;
@@ -782,7 +786,9 @@ template <class P, int QM>
 __global__ void __launch_bounds__(kWarps * 32, ColGeo<P>::kMinBlocksA) k_col_a(const SpecArgs a, int nxt) {
   extern __shared__ float2 smem[];
   ColCtx<P> c(a, smem, nxt);
+  chain_next();
   load_stage_tw<P>(c.tw, a.twy);
+  chain_wait();
   cols_to_tile<P>(c.tile, a.t1, a, c.b, c.x0);
   __syncthreads();
   // The zeroth Born order's filter (|k| / w)^0 is the identity: its output is the
@@ -853,7 +859,9 @@ __global__ void __launch_bounds__(kWarps * 32, ColGeo<P>::kMinBlocks) k_col_b(co
   ColCtx<P> c(a, smem, nxt);
   float2* tiles[2] = {c.tile, c.tw + tw_size<P>()};
   const long long lineoff = (long long)c.col * ColGeo<P>::LINE;
+  chain_next();
   load_stage_tw<P>(c.tw, a.twy);
+  chain_wait();
   const int xq = c.x < a.d.NX ? c.x : 0;
   float2 acc[P::E];
 #pragma unroll
@@ -962,7 +970,9 @@ __global__ void __launch_bounds__(kWarps * 32, ColGeo<P>::kMinBlocks)
     tma::mbar_init(&bar[1], 1);
     tma::fence_mbar_init();
   }
+  chain_next();
   load_stage_tw<P>(tw, a.twy);
+  chain_wait();
   __syncthreads();
   auto issue = [&](int term, int buf) {
     tma::mbar_expect_tx(&bar[buf], (unsigned)((C::TILE + qt) * sizeof(float2)));
@@ -1082,7 +1092,9 @@ __global__ void __launch_bounds__(kWarps * 32, col_a_tma_min_blocks<P>(kQT))
     tma::mbar_init(&bar[2], 1);
     tma::fence_mbar_init();
   }
+  chain_next();
   load_stage_tw<P>(tw, a.twy);
+  chain_wait();
   __syncthreads();
   auto issue_q = [&](int term) {  // the phase tile of `term` into slot term & 1
     uint64_t* qb = &bar[1 + (term & 1)];
@@ -1269,8 +1281,7 @@ cudaError_t launch_hinted(K kernel, unsigned grid, size_t sm, cudaStream_t s, co
     const int res = resident_ctas(kernel, sm);
     if (res > 0 && grid > (unsigned)res) b.pf_ctas = res;
   }
-  kernel<<<grid, kWarps * 32, sm, s>>>(b, args...);
-  return cudaSuccess;
+  return launch_chained(a.d.chained, kernel, grid, kWarps * 32, sm, s, b, args...);
 }
 
 template <class P>
@@ -1369,7 +1380,7 @@ cudaError_t col_type_a_tma(const SpecArgs& a, int qmode, cudaStream_t s) {
   if (e != cudaSuccess) return e;
 #define FWIX_FAST_CAT(Q, QT)                                                                          \
   e = opt_in_smem(k_col_a_tma<P, Q, QT>, sm);                                                         \
-  if (e == cudaSuccess) k_col_a_tma<P, Q, QT><<<grid, kWarps * 32, sm, s>>>(a, nxt, tin, tout, tq);
+  if (e == cudaSuccess) e = launch_chained(a.d.chained, k_col_a_tma<P, Q, QT>, grid, kWarps * 32, sm, s, a, nxt, tin, tout, tq);
   switch (qmode) {
     case Q_PS_FWD:
       if (qtile) {
@@ -1406,7 +1417,7 @@ cudaError_t col_type_a(const SpecArgs& a, int qmode, cudaStream_t s) {
 #define FWIX_FAST_CA(Q)                                                           \
   case Q:                                                                         \
     e = opt_in_smem(k_col_a<P, Q>, sm);                                           \
-    if (e == cudaSuccess) k_col_a<P, Q><<<grid, kWarps * 32, sm, s>>>(a, nxt);    \
+    if (e == cudaSuccess) e = launch_chained(a.d.chained, k_col_a<P, Q>, grid, kWarps * 32, sm, s, a, nxt); \
     break;
   switch (qmode) {
     FWIX_FAST_CA(Q_PS_FWD)
@@ -1437,7 +1448,7 @@ cudaError_t col_type_b_tma(const SpecArgs& a, int qmode, cudaStream_t s) {
   if (e != cudaSuccess) return e;
 #define FWIX_FAST_CBT(Q, QT)                                                                          \
   e = opt_in_smem(k_col_b_tma<P, Q, QT>, sm);                                                         \
-  if (e == cudaSuccess) k_col_b_tma<P, Q, QT><<<grid, kWarps * 32, sm, s>>>(a, nxt, tin, tout, tq);
+  if (e == cudaSuccess) e = launch_chained(a.d.chained, k_col_b_tma<P, Q, QT>, grid, kWarps * 32, sm, s, a, nxt, tin, tout, tq);
   switch (qmode) {
     case Q_PS_FWD:
       if (qtile) {
@@ -1474,7 +1485,7 @@ cudaError_t col_type_b(const SpecArgs& a, int qmode, cudaStream_t s) {
 #define FWIX_FAST_CB(Q)                                                           \
   case Q:                                                                         \
     e = opt_in_smem(k_col_b<P, Q>, sm);                                           \
-    if (e == cudaSuccess) k_col_b<P, Q><<<grid, kWarps * 32, sm, s>>>(a, nxt);    \
+    if (e == cudaSuccess) e = launch_chained(a.d.chained, k_col_b<P, Q>, grid, kWarps * 32, sm, s, a, nxt); \
     break;
   switch (qmode) {
     FWIX_FAST_CB(Q_PS_FWD)

@@ -304,6 +304,9 @@ __global__ void __launch_bounds__(S::ROW_THREADS, min_blocks<S>(S::ROW_THREADS, 
   float2* const buf1 = buf0 + d.rows() * row_ls(d.n(), S::RT);
   const RowCtx<S> c(a, d);
   const RowPlace<S, false> w(d);
+  chain_next();
+  fill_twiddles(tw, a.twx, RT, d.rb(), d.ra(), d.row_threads());
+  chain_wait();
   constexpr bool kSmooth = CLS == C_SMOOTH;
   __shared__ typename std::conditional<kSmooth, HatTables, int>::type hat;
   float unit = 0.f;
@@ -311,7 +314,6 @@ __global__ void __launch_bounds__(S::ROW_THREADS, min_blocks<S>(S::ROW_THREADS, 
     unit = phase_unit(a, c.iw);
     stage_hat(hat, a, c.iw, unit);
   }
-  fill_twiddles(tw, a.twx, RT, d.rb(), d.ra(), d.row_threads());
   const long long roff = (c.b * a.d.NY + (c.live ? c.y : 0)) * d.n();
   float2 raw[RT];
 #pragma unroll
@@ -439,6 +441,9 @@ __global__ void __launch_bounds__(S::ROW_THREADS, min_blocks<S>(S::ROW_THREADS, 
   float2* const buf1 = buf0 + d.rows() * row_ls(d.n(), d.ra());
   const RowCtx<S> c(a, d);
   const RowPlace<S, true> w(d);
+  chain_next();
+  fill_twiddles(tw, a.twx, d.ra(), d.rb(), RT, d.row_threads());
+  chain_wait();
   // kDeriv: the sum of w_r' C_r T_r beside the step's own
   constexpr bool kDeriv = CLS == C_PAIR || CLS == C_DERIV, kSmooth = CLS == C_SMOOTH || kDeriv;
   __shared__ typename std::conditional<kSmooth, HatTables, int>::type hat;
@@ -447,7 +452,6 @@ __global__ void __launch_bounds__(S::ROW_THREADS, min_blocks<S>(S::ROW_THREADS, 
     unit = phase_unit(a, c.iw);
     stage_hat(hat, a, c.iw, unit);
   }
-  fill_twiddles(tw, a.twx, d.ra(), d.rb(), RT, d.row_threads());
   float2 acc[RT];
   float2 acc2[kDeriv ? RT : 1];
 #pragma unroll
@@ -725,7 +729,9 @@ __global__ void __launch_bounds__(S::COL_THREADS, min_blocks<S>(S::COL_THREADS))
   float2* const buf0 = sm + d.fwd_rows_tw() + d.inv_rows_tw();
   float2* const buf1 = buf0 + (d.n() << d.sh());
   const ColCtx<S> c(a, d);
+  chain_next();
   col_twiddles(a, d, tw);
+  chain_wait();
   // the zeroth Born order's filter is the identity: its output is the input,
   // scaled as the transform pair would
   const int first = qm == Q_KPOW && a.term0 == 0 ? 1 : 0;
@@ -773,7 +779,9 @@ __global__ void __launch_bounds__(S::COL_THREADS, min_blocks<S>(S::COL_THREADS))
   float2* const buf0 = sm + d.fwd_rows_tw() + d.inv_rows_tw();
   float2* const buf1 = buf0 + (d.n() << d.sh());
   const ColCtx<S> c(a, d);
+  chain_next();
   col_twiddles(a, d, tw);
+  chain_wait();
   float2 acc[RT];
 #pragma unroll
   for (int r = 0; r < RT; ++r) acc[r] = make_float2(0.f, 0.f);
@@ -822,7 +830,9 @@ __global__ void __launch_bounds__(S::COL_THREADS, min_blocks<S>(S::COL_THREADS))
   float2* const buf0 = sm + d.fwd_rows_tw() + d.inv_rows_tw();
   float2* const buf1 = buf0 + (d.n() << d.sh());
   const ColCtx<S> c(a, d);
+  chain_next();
   col_twiddles(a, d, tw);
+  chain_wait();
   const long long off = c.b * a.d.slice + c.x;
   float2 v[RT];
   if (!INV) {
@@ -920,12 +930,12 @@ cudaError_t opt_in(K kernel, size_t bytes) {
 }
 
 template <class K, class... Args>
-cudaError_t launch(K kernel, unsigned grid, unsigned threads, size_t smem, cudaStream_t s, Args... args) {
+cudaError_t launch(K kernel, unsigned grid, unsigned threads, size_t smem, cudaStream_t s, const SpecArgs& a,
+                   Args... args) {
   cudaError_t e = opt_in(kernel, smem);
-  if (e != cudaSuccess) return e;
-  kernel<<<grid, threads, smem, s>>>(args...);
-  count_launch();
-  return cudaGetLastError();
+  if (e == cudaSuccess) e = launch_chained(a.d.chained, kernel, grid, threads, smem, s, a, args...);
+  if (e == cudaSuccess) count_launch();
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 template <class S>

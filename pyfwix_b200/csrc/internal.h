@@ -54,6 +54,7 @@ struct Dims {
   int nw, ns;       // frequencies, shots
   long long slice;  // NX * NY
   long long wfld;   // ns * nw * NX * NY
+  int chained;      // launch kernels with launch_chained's early start
 };
 
 // Everything a spectral kernel may read.  Passed by value (kernel parameter).
@@ -143,6 +144,38 @@ struct SpecArgs {
   // once every resident CTA has run (0: none)
   int pf_ctas;
 };
+
+// Chained launches.  A kernel launched with chained set may start, CTA by CTA, while
+// the kernel before it on the stream drains: up to chain_wait() it may only touch
+// what no kernel on the stream writes (a plan's twiddle tables, its own shared
+// memory); chain_wait() returns once the kernel before it has completed with its
+// writes visible (at once for an ordinary launch).  Every thread calls both,
+// chain_next() first.  The prologue and the launch gap (1 - 2 us of kernels of 5 -
+// 30 us at 128 x 128 and below) then go under the kernel before: modelling at 128 x
+// 128 x 64 2432 -> 2042 us, an NSPS step and its adjoint at 105 x 90 x 24 59 -> 46
+// us, the Born pair at 256 x 256 x 128 13.71 -> 13.35 ms.  Instances that share the
+// GPU over several streams are not chained (fwix_sweep): there the waiting CTAs hold
+// places that the other streams' kernels could use (6.31 -> 6.48 ms, four shots).
+#ifdef __CUDACC__
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <class... KArgs, class... Args>
+cudaError_t launch_chained(bool chained, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                           Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = chained ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+#endif
 
 // Spectral passes (dispatch.cu: register-resident passes for lengths with a
 // compile-time plan (fast.cuh) or a run-time one (flex.cuh), the generic per-warp

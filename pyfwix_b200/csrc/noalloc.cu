@@ -132,7 +132,7 @@ extern "C" fwix_status fwix_step_noalloc(const fwix_desc* desc, int kind, int iz
   if (iz < 0 || iz >= q.nz) return fail(FWIX_ERR_INVALID, "depth index out of range");
   if ((long long)q.nx + q.padx > FWIX_MAX_N || (long long)q.ny + q.pady > FWIX_MAX_N)
     return fail(FWIX_ERR_UNSUPPORTED, "wavefield sizes must be 2^a 3^b 5^c 7^d and at most 1024");
-  fwix::Dims d;
+  fwix::Dims d = {};  // (its tables are written on the stream: not chained)
   d.nx = q.nx;
   d.ny = q.ny;
   d.NX = q.nx + q.padx;

@@ -76,6 +76,8 @@ __global__ void __launch_bounds__(kCells * kGroups)
     k_reflect(Dims d, int adjoint, const float2* __restrict__ s0, const float2* __restrict__ s1,
               const float2* __restrict__ r0, const float2* __restrict__ r1, long long mw,
               const float2* __restrict__ in, float2* __restrict__ out) {
+  chain_next();
+  chain_wait();
   const Cell c = this_cell(d);
   // one model for every frequency: the first group forms each cell's coefficient once
   __shared__ float2 rs[kCells];
@@ -106,6 +108,8 @@ __global__ void __launch_bounds__(kCells * kGroups)
 __global__ void __launch_bounds__(kCells * kGroups)
     k_ic_fwd(Dims d, const float2* __restrict__ bg, const float2* __restrict__ image, long long img_w,
              float2* __restrict__ wfld) {
+  chain_next();
+  chain_wait();
   const Cell c = this_cell(d);
   if (!c.ok) return;
 #pragma unroll 4
@@ -124,6 +128,8 @@ template <bool S1>
 __global__ void __launch_bounds__(kCells * kGroups)
     k_ic_adj(Dims d, const float2* __restrict__ bg, const float2* __restrict__ wfld, float2* __restrict__ image,
              int add, int wsum) {
+  chain_next();
+  chain_wait();
   const Cell c = this_cell(d);
   float2 acc[1] = {make_float2(0.f, 0.f)};
   const int ns = S1 ? 1 : d.ns;
@@ -183,6 +189,8 @@ __global__ void __launch_bounds__(kCells * kGroups)
                   float2* dm1, float2* dm2, float2* dm3, long long dm_w, float2* dr, int add,
                   const float2* __restrict__ bg, float2* __restrict__ wf, const float2* __restrict__ bg2,
                   const float2* __restrict__ wf2) {
+  chain_next();
+  chain_wait();
   const Cell c = this_cell(d);
   const int ns = S1 ? 1 : d.ns;
   const long long plane = (long long)d.ny * d.nx;
@@ -301,6 +309,8 @@ __global__ void __launch_bounds__(256)
                  const float2* __restrict__ r0, const float2* __restrict__ r1, const float2* __restrict__ dm0,
                  const float2* __restrict__ dm1, const float2* __restrict__ dm2, const float2* __restrict__ dm3,
                  float2* __restrict__ tab) {
+  chain_next();
+  chain_wait();
   const long long n = (long long)d.ny * d.nx;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {
@@ -319,6 +329,8 @@ template <bool S1>
 __global__ void __launch_bounds__(kCells * kGroups)
     k_image_acc(Dims d, const float2* __restrict__ S, const float2* __restrict__ R, float* __restrict__ img,
                 int add) {
+  chain_next();
+  chain_wait();
   const Cell c = this_cell(d);
   float2 acc[1] = {make_float2(0.f, 0.f)};
   const int ns = S1 ? 1 : d.ns;
@@ -340,6 +352,8 @@ template <bool S1>
 __global__ void __launch_bounds__(kCells * kGroups)
     k_image_acc2(Dims d, int ny2, int nx2, const float2* __restrict__ S, const float2* __restrict__ R1,
                  const float2* __restrict__ R2, float* __restrict__ img1, float* __restrict__ img2, int add) {
+  chain_next();
+  chain_wait();
   const Cell c = this_cell(d);
   float2 acc[1] = {make_float2(0.f, 0.f)};
   const int ns = S1 ? 1 : d.ns;
@@ -380,6 +394,8 @@ __global__ void k_axpy(long long n, const float2* __restrict__ x, float2* __rest
 // wfld[shot, w, y, x] += sum_k weight_k * traces[trace_k, w] for each listed cell.
 __global__ void __launch_bounds__(256) k_inject(Dims d, InjectLevel L, const float2* __restrict__ traces,
                                                 float2* wfld) {
+  chain_next();
+  chain_wait();
   __shared__ float2 tile[32][33];
   const int e0 = blockIdx.x * 32, w0 = blockIdx.y * 32;
   const int iw = w0 + threadIdx.x;
@@ -405,6 +421,8 @@ __global__ void __launch_bounds__(256) k_inject(Dims d, InjectLevel L, const flo
 // traces[t, w] += sum of the four corner weights times the wavefield.
 __global__ void __launch_bounds__(256) k_record(Dims d, InjectLevel L, const float2* __restrict__ wfld,
                                                 float2* traces) {
+  chain_next();
+  chain_wait();
   __shared__ float2 tile[32][33];
   const int e0 = blockIdx.x * 32, w0 = blockIdx.y * 32;
   const int e = e0 + threadIdx.x;
@@ -435,117 +453,134 @@ __global__ void __launch_bounds__(256) k_record(Dims d, InjectLevel L, const flo
 cudaError_t launch_reflect(const Dims& d, int adjoint, const float2* s0, const float2* s1,
                            const float2* r0, const float2* r1, long long mw, const float2* in,
                            float2* out, int add, cudaStream_t s) {
+  cudaError_t e = cudaSuccess;
   if (!add) {
-    cudaError_t e = cudaMemsetAsync(out, 0, d.wfld * sizeof(float2), s);
+    e = cudaMemsetAsync(out, 0, d.wfld * sizeof(float2), s);
     if (e != cudaSuccess) return e;
   }
   if (d.ns == 1)
-    k_reflect<true><<<cell_blocks(d), dim3(kCells, kGroups), 0, s>>>(d, adjoint, s0, s1, r0, r1, mw, in, out);
+    e = launch_chained(d.chained, k_reflect<true>, cell_blocks(d), dim3(kCells, kGroups), 0, s,
+                       d, adjoint, s0, s1, r0, r1, mw, in, out);
   else
-    k_reflect<false><<<cell_blocks(d), dim3(kCells, kGroups), 0, s>>>(d, adjoint, s0, s1, r0, r1, mw, in, out);
-  count_launch();
-  return cudaGetLastError();
+    e = launch_chained(d.chained, k_reflect<false>, cell_blocks(d), dim3(kCells, kGroups), 0, s,
+                       d, adjoint, s0, s1, r0, r1, mw, in, out);
+  if (e == cudaSuccess) count_launch();
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 cudaError_t launch_ic_fwd(const Dims& d, const float2* bg, const float2* image, long long img_w,
                           float2* wfld, int add, cudaStream_t s) {
+  cudaError_t e = cudaSuccess;
   if (!add) {
-    cudaError_t e = cudaMemsetAsync(wfld, 0, d.wfld * sizeof(float2), s);
+    e = cudaMemsetAsync(wfld, 0, d.wfld * sizeof(float2), s);
     if (e != cudaSuccess) return e;
   }
-  k_ic_fwd<<<cell_blocks(d), dim3(kCells, kGroups), 0, s>>>(d, bg, image, img_w, wfld);
-  count_launch();
-  return cudaGetLastError();
+  e = launch_chained(d.chained, k_ic_fwd, cell_blocks(d), dim3(kCells, kGroups), 0, s, d, bg, image, img_w, wfld);
+  if (e == cudaSuccess) count_launch();
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 cudaError_t launch_ic_adj(const Dims& d, const float2* bg, const float2* wfld, float2* image,
                           long long img_w, int add, cudaStream_t s) {
+  cudaError_t e = cudaSuccess;
   if (d.ns == 1)
-    k_ic_adj<true><<<cell_blocks(d), dim3(kCells, kGroups), 0, s>>>(d, bg, wfld, image, add, img_w == 0);
+    e = launch_chained(d.chained, k_ic_adj<true>, cell_blocks(d), dim3(kCells, kGroups), 0, s,
+                       d, bg, wfld, image, add, img_w == 0);
   else
-    k_ic_adj<false><<<cell_blocks(d), dim3(kCells, kGroups), 0, s>>>(d, bg, wfld, image, add, img_w == 0);
-  count_launch();
-  return cudaGetLastError();
+    e = launch_chained(d.chained, k_ic_adj<false>, cell_blocks(d), dim3(kCells, kGroups), 0, s,
+                       d, bg, wfld, image, add, img_w == 0);
+  if (e == cudaSuccess) count_launch();
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 cudaError_t launch_lin_reflect(const Dims& d, int adjoint, const float2* s0, const float2* s1,
                                const float2* r0, const float2* r1, long long mw, float2* dm0,
                                float2* dm1, float2* dm2, float2* dm3, long long dm_w, float2* dr,
                                int add, cudaStream_t s) {
-  k_lin_reflect<false, false, false><<<cell_blocks(d), dim3(kCells, kGroups), 0, s>>>(
-      d, adjoint, s0, s1, r0, r1, mw, dm0, dm1, dm2, dm3, dm_w, dr, add, nullptr, nullptr, nullptr, nullptr);
-  count_launch();
-  return cudaGetLastError();
+  cudaError_t e = launch_chained(d.chained, k_lin_reflect<false, false, false>, cell_blocks(d), dim3(kCells, kGroups), 0, s,
+                     d, adjoint, s0, s1, r0, r1, mw, dm0, dm1, dm2, dm3, dm_w, dr, add, nullptr, nullptr, nullptr,
+                     nullptr);
+  if (e == cudaSuccess) count_launch();
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 cudaError_t launch_lin_reflect_ic(const Dims& d, int adjoint, const float2* s0, const float2* s1,
                                   const float2* r0, const float2* r1, long long mw, float2* dm0, float2* dm1,
                                   float2* dm2, float2* dm3, long long dm_w, const float2* bg, float2* wf, int add,
                                   cudaStream_t s, const float2* bg2, const float2* wf2) {
+  cudaError_t e = cudaSuccess;
   const dim3 grid(cell_blocks(d)), block(kCells, kGroups);
   if (wf2) {
     if (!adjoint || mw != 0 || dm_w != 0 || !bg2) return cudaErrorInvalidValue;
     if (d.ns == 1)
-      k_lin_reflect<true, true, true><<<grid, block, 0, s>>>(d, adjoint, s0, s1, r0, r1, mw, dm0, dm1, dm2, dm3,
-                                                             dm_w, nullptr, add, bg, wf, bg2, wf2);
+      e = launch_chained(d.chained, k_lin_reflect<true, true, true>, grid, block, 0, s,
+                         d, adjoint, s0, s1, r0, r1, mw, dm0, dm1, dm2, dm3, dm_w, nullptr, add, bg, wf, bg2, wf2);
     else
-      k_lin_reflect<true, false, true><<<grid, block, 0, s>>>(d, adjoint, s0, s1, r0, r1, mw, dm0, dm1, dm2, dm3,
-                                                              dm_w, nullptr, add, bg, wf, bg2, wf2);
+      e = launch_chained(d.chained, k_lin_reflect<true, false, true>, grid, block, 0, s,
+                         d, adjoint, s0, s1, r0, r1, mw, dm0, dm1, dm2, dm3, dm_w, nullptr, add, bg, wf, bg2, wf2);
   } else if (d.ns == 1) {
-    k_lin_reflect<true, true, false><<<grid, block, 0, s>>>(d, adjoint, s0, s1, r0, r1, mw, dm0, dm1, dm2, dm3,
-                                                            dm_w, nullptr, add, bg, wf, nullptr, nullptr);
+    e = launch_chained(d.chained, k_lin_reflect<true, true, false>, grid, block, 0, s,
+                       d, adjoint, s0, s1, r0, r1, mw, dm0, dm1, dm2, dm3, dm_w, nullptr, add, bg, wf, nullptr,
+                       nullptr);
   } else {
-    k_lin_reflect<true, false, false><<<grid, block, 0, s>>>(d, adjoint, s0, s1, r0, r1, mw, dm0, dm1, dm2, dm3,
-                                                             dm_w, nullptr, add, bg, wf, nullptr, nullptr);
+    e = launch_chained(d.chained, k_lin_reflect<true, false, false>, grid, block, 0, s,
+                       d, adjoint, s0, s1, r0, r1, mw, dm0, dm1, dm2, dm3, dm_w, nullptr, add, bg, wf, nullptr,
+                       nullptr);
   }
-  count_launch();
-  return cudaGetLastError();
+  if (e == cudaSuccess) count_launch();
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 cudaError_t launch_refl_table(const Dims& d, int adjoint, const float2* s0, const float2* s1, const float2* r0,
                               const float2* r1, const float2* dm0, const float2* dm1, const float2* dm2,
                               const float2* dm3, float2* tab, cudaStream_t s) {
-  k_refl_table<<<grid1d((long long)d.ny * d.nx), 256, 0, s>>>(d, adjoint, s0, s1, r0, r1, dm0, dm1, dm2, dm3, tab);
-  count_launch();
-  return cudaGetLastError();
+  cudaError_t e = launch_chained(d.chained, k_refl_table, grid1d((long long)d.ny * d.nx), 256, 0, s,
+                     d, adjoint, s0, s1, r0, r1, dm0, dm1, dm2, dm3, tab);
+  if (e == cudaSuccess) count_launch();
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 cudaError_t launch_image_acc(const Dims& d, const float2* S, const float2* R, float* img, int add,
                              cudaStream_t s) {
+  cudaError_t e = cudaSuccess;
   if (d.ns == 1)
-    k_image_acc<true><<<cell_blocks(d), dim3(kCells, kGroups), 0, s>>>(d, S, R, img, add);
+    e = launch_chained(d.chained, k_image_acc<true>, cell_blocks(d), dim3(kCells, kGroups), 0, s, d, S, R, img, add);
   else
-    k_image_acc<false><<<cell_blocks(d), dim3(kCells, kGroups), 0, s>>>(d, S, R, img, add);
-  count_launch();
-  return cudaGetLastError();
+    e = launch_chained(d.chained, k_image_acc<false>, cell_blocks(d), dim3(kCells, kGroups), 0, s, d, S, R, img, add);
+  if (e == cudaSuccess) count_launch();
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 cudaError_t launch_correlate_padded(const Dims& d, const float2* S, const float2* R, float* img, int add,
                                     cudaStream_t s) {
+  cudaError_t e = cudaSuccess;
   Dims full = d;  // iterate over the padded slice: the cell window is the whole NY x NX
   full.nx = d.NX;
   full.ny = d.NY;
   if (d.ns == 1)
-    k_image_acc<true><<<cell_blocks(full), dim3(kCells, kGroups), 0, s>>>(full, S, R, img, add);
+    e = launch_chained(d.chained, k_image_acc<true>, cell_blocks(full), dim3(kCells, kGroups), 0, s,
+                       full, S, R, img, add);
   else
-    k_image_acc<false><<<cell_blocks(full), dim3(kCells, kGroups), 0, s>>>(full, S, R, img, add);
-  count_launch();
-  return cudaGetLastError();
+    e = launch_chained(d.chained, k_image_acc<false>, cell_blocks(full), dim3(kCells, kGroups), 0, s,
+                       full, S, R, img, add);
+  if (e == cudaSuccess) count_launch();
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 cudaError_t launch_correlate2_padded(const Dims& d, const float2* S, const float2* R1, const float2* R2,
                                      float* img1, float* img2, int add, cudaStream_t s) {
+  cudaError_t e = cudaSuccess;
   Dims full = d;  // the padded slice; img2 covers the model window d.ny x d.nx
   full.nx = d.NX;
   full.ny = d.NY;
   if (d.ns == 1)
-    k_image_acc2<true><<<cell_blocks(full), dim3(kCells, kGroups), 0, s>>>(full, d.ny, d.nx, S, R1, R2, img1, img2,
-                                                                           add);
+    e = launch_chained(d.chained, k_image_acc2<true>, cell_blocks(full), dim3(kCells, kGroups), 0, s,
+                       full, d.ny, d.nx, S, R1, R2, img1, img2, add);
   else
-    k_image_acc2<false><<<cell_blocks(full), dim3(kCells, kGroups), 0, s>>>(full, d.ny, d.nx, S, R1, R2, img1,
-                                                                            img2, add);
-  count_launch();
-  return cudaGetLastError();
+    e = launch_chained(d.chained, k_image_acc2<false>, cell_blocks(full), dim3(kCells, kGroups), 0, s,
+                       full, d.ny, d.nx, S, R1, R2, img1, img2, add);
+  if (e == cudaSuccess) count_launch();
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 cudaError_t launch_axpy(long long n, const float2* x, float2* y, cudaStream_t s) {
@@ -556,20 +591,22 @@ cudaError_t launch_axpy(long long n, const float2* x, float2* y, cudaStream_t s)
 
 cudaError_t launch_inject(const Dims& d, const InjectLevel& L, const float2* traces, float2* wfld,
                           cudaStream_t s) {
+  cudaError_t e = cudaSuccess;
   if (L.ncell == 0) return cudaSuccess;
   const dim3 grid((unsigned)((L.ncell + 31) / 32), (unsigned)((d.nw + 31) / 32));
-  k_inject<<<grid, dim3(32, 8), 0, s>>>(d, L, traces, wfld);
-  count_launch();
-  return cudaGetLastError();
+  e = launch_chained(d.chained, k_inject, grid, dim3(32, 8), 0, s, d, L, traces, wfld);
+  if (e == cudaSuccess) count_launch();
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 cudaError_t launch_record(const Dims& d, const InjectLevel& L, const float2* wfld, float2* traces,
                           cudaStream_t s) {
+  cudaError_t e = cudaSuccess;
   if (L.ntr == 0) return cudaSuccess;
   const dim3 grid((unsigned)((L.ntr + 31) / 32), (unsigned)((d.nw + 31) / 32));
-  k_record<<<grid, dim3(32, 8), 0, s>>>(d, L, wfld, traces);
-  count_launch();
-  return cudaGetLastError();
+  e = launch_chained(d.chained, k_record, grid, dim3(32, 8), 0, s, d, L, wfld, traces);
+  if (e == cudaSuccess) count_launch();
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 }  // namespace fwix

@@ -419,6 +419,8 @@ __global__ void k_phase_shift(const SpecArgs a, const float2* __restrict__ in, f
 
 template <int W>
 __global__ void k_weight(const SpecArgs a, int t, const float2* __restrict__ in, float2* out, int add) {
+  chain_next();
+  chain_wait();
   const long long n = a.d.wfld;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {
@@ -458,6 +460,8 @@ cudaError_t launch_phase_shift(const SpecArgs& a, int mode, const float2* sref_w
 // Forward phase factors x norm of one depth for every (ref, w, |kx|, |ky|): the
 // same arithmetic as the in-kernel evaluation (k depends on |index| only).
 __global__ void k_phase_table(const SpecArgs a, float2* dst) {
+  chain_next();
+  chain_wait();
   const long long n = (long long)a.nterm * a.d.nw * a.ptab_nx * a.ptab_ny;
   SpecArgs b = a;
   b.ptab = nullptr;
@@ -478,9 +482,9 @@ __global__ void k_phase_table(const SpecArgs a, float2* dst) {
 
 cudaError_t launch_phase_table(const SpecArgs& a, float2* dst, cudaStream_t s) {
   const long long n = (long long)a.nterm * a.d.nw * a.ptab_nx * a.ptab_ny;
-  k_phase_table<<<grid1d(n), 256, 0, s>>>(a, dst);
-  count_launch();
-  return cudaGetLastError();
+  const cudaError_t e = launch_chained(a.d.chained, k_phase_table, grid1d(n), 256, 0, s, a, dst);
+  if (e == cudaSuccess) count_launch();
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 cudaError_t launch_select(const SpecArgs& a, int value, const float2* in, float2* out, int add,
@@ -491,6 +495,8 @@ cudaError_t launch_select(const SpecArgs& a, int value, const float2* in, float2
 }
 
 __global__ void k_scat_table(const SpecArgs a, float2* dst) {
+  chain_next();
+  chain_wait();
   const long long n = (long long)a.nterm * a.d.slice;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     const int t = (int)(i / a.d.slice);
@@ -501,15 +507,17 @@ __global__ void k_scat_table(const SpecArgs a, float2* dst) {
 }
 
 cudaError_t launch_scat_table(const SpecArgs& a, float2* dst, cudaStream_t s) {
-  k_scat_table<<<grid1d((long long)a.nterm * a.d.slice), 256, 0, s>>>(a, dst);
-  count_launch();
-  return cudaGetLastError();
+  const cudaError_t e =
+      launch_chained(a.d.chained, k_scat_table, grid1d((long long)a.nterm * a.d.slice), 256, 0, s, a, dst);
+  if (e == cudaSuccess) count_launch();
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 cudaError_t launch_taper(const SpecArgs& a, const float2* in, float2* out, int add, cudaStream_t s) {
-  k_weight<W_TAPER><<<grid1d(a.d.wfld), 256, 0, s>>>(a, 0, in, out, add);
-  count_launch();
-  return cudaGetLastError();
+  const cudaError_t e =
+      launch_chained(a.d.chained, k_weight<W_TAPER>, grid1d(a.d.wfld), 256, 0, s, a, 0, in, out, add);
+  if (e == cudaSuccess) count_launch();
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 }  // namespace fwix
