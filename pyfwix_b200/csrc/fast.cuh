@@ -781,6 +781,23 @@ __device__ __forceinline__ void col_factors(const SpecArgs& a, int t, int iw, in
   }
 }
 
+// The Born filter of term t at this lane's spectrum samples (real factors).
+template <class P>
+__device__ __forceinline__ void kpow_factors(const SpecArgs& a, int t, int iw, int x, int lane_t, float (&f)[P::E]) {
+  const KPow k(a, t, iw, x);
+  if (k.n == 1) {  // the usual order, without the power loop
+#pragma unroll
+    for (int e = 0; e < P::E; ++e) {
+      const int y = pos_last<P>(lane_t, e);
+      const float ky = (float)min(y, P::N - y) * k.dk;
+      f[e] = (k.kx2 + ky * ky) * k.s;
+    }
+  } else {
+#pragma unroll
+    for (int e = 0; e < P::E; ++e) f[e] = k.at(pos_last<P>(lane_t, e));
+  }
+}
+
 // t2[term] = F_y^-1(Q_term * F_y(t1[0])); the spectrum stays in registers.
 template <class P, int QM>
 __global__ void __launch_bounds__(kWarps * 32, ColGeo<P>::kMinBlocksA) k_col_a(const SpecArgs a, int nxt) {
@@ -811,7 +828,7 @@ __global__ void __launch_bounds__(kWarps * 32, ColGeo<P>::kMinBlocksA) k_col_a(c
   // current term is transformed; with 16 the spectrum, the term and the factors
   // do not fit the two-CTA register budget together, so each term's factors are
   // fetched as they are applied.
-  constexpr bool kPrefetch = P::E <= 12;
+  constexpr bool kPrefetch = P::E <= 12 && QM != Q_KPOW;
   float2 q[kPrefetch ? P::E : 1];
   if constexpr (kPrefetch) col_factors<P, QM>(a, first, c.iw, xq, c.t, q);
   for (int term = first; term < a.nterm; ++term) {
@@ -820,6 +837,11 @@ __global__ void __launch_bounds__(kWarps * 32, ColGeo<P>::kMinBlocksA) k_col_a(c
 #pragma unroll
       for (int e = 0; e < P::E; ++e) v[e] = cmul(psi[e], q[e]);
       if (term + 1 < a.nterm) col_factors<P, QM>(a, term + 1, c.iw, xq, c.t, q);
+    } else if constexpr (QM == Q_KPOW) {
+      float f[P::E];
+      kpow_factors<P>(a, term, c.iw, xq, c.t, f);
+#pragma unroll
+      for (int e = 0; e < P::E; ++e) v[e] = cscale(psi[e], f[e]);
     } else {
       col_factors<P, QM>(a, term, c.iw, xq, c.t, v);
 #pragma unroll
@@ -875,16 +897,23 @@ __global__ void __launch_bounds__(kWarps * 32, ColGeo<P>::kMinBlocks) k_col_b(co
     } else {
       cp_async_wait<0>();
     }
-    float2 q[P::E];
-    col_factors<P, QM>(a, term, c.iw, xq, c.t, q);
+    float2 q[QM == Q_KPOW ? 1 : P::E];
+    if constexpr (QM != Q_KPOW) col_factors<P, QM>(a, term, c.iw, xq, c.t, q);
     __syncthreads();  // this term's tile is complete
     float2* line = tiles[term & 1] + lineoff;
     float2 v[P::E];
 #pragma unroll
     for (int e = 0; e < P::E; ++e) v[e] = line[swz(pos_first<P>(c.t, e))];
     fft_fwd<P>(v, c.t, c.tw, line);
+    if constexpr (QM == Q_KPOW) {
+      float f[P::E];
+      kpow_factors<P>(a, term, c.iw, xq, c.t, f);
 #pragma unroll
-    for (int e = 0; e < P::E; ++e) acc[e] = cadd(acc[e], cmul(v[e], q[e]));
+      for (int e = 0; e < P::E; ++e) acc[e] = cfma(v[e], f[e], acc[e]);
+    } else {
+#pragma unroll
+      for (int e = 0; e < P::E; ++e) acc[e] = cadd(acc[e], cmul(v[e], q[e]));
+    }
   }
   __syncthreads();
   fft_inv<P>(acc, c.t, c.tw, c.line);
@@ -988,8 +1017,9 @@ __global__ void __launch_bounds__(kWarps * 32, ColGeo<P>::kMinBlocks)
   for (int term = 0; term < a.nterm; ++term) {
     const int buf = term & 1;
     if (threadIdx.x == 0 && term + 1 < a.nterm) issue(term + 1, buf ^ 1);
-    float2 q[kQT ? 1 : P::E];
-    if constexpr (!kQT) col_factors<P, QM>(a, term, iw, xq, t, q);
+    constexpr bool kQ = !kQT && QM != Q_KPOW;
+    float2 q[kQ ? P::E : 1];
+    if constexpr (kQ) col_factors<P, QM>(a, term, iw, xq, t, q);
     const bool ok = tma::mbar_wait(&bar[buf], (unsigned)(term >> 1) & 1u);
     if (!__syncthreads_and(ok)) {
       if (threadIdx.x == 0) {
@@ -1012,6 +1042,11 @@ __global__ void __launch_bounds__(kWarps * 32, ColGeo<P>::kMinBlocks)
         const float2 f = qr[min(ky, P::N - ky)];
         acc[e] = cadd(acc[e], cmul(v[e], flip ? cconj(f) : f));
       }
+    } else if constexpr (QM == Q_KPOW) {
+      float f[P::E];
+      kpow_factors<P>(a, term, iw, xq, t, f);
+#pragma unroll
+      for (int e = 0; e < P::E; ++e) acc[e] = cfma(v[e], f[e], acc[e]);
     } else {
 #pragma unroll
       for (int e = 0; e < P::E; ++e) acc[e] = cadd(acc[e], cmul(v[e], q[e]));
@@ -1175,6 +1210,11 @@ __global__ void __launch_bounds__(kWarps * 32, col_a_tma_min_blocks<P>(kQT))
         const float2 f = qr[min(ky, P::N - ky)];
         v[e] = cmul(psi[e], flip ? cconj(f) : f);
       }
+    } else if constexpr (QM == Q_KPOW) {
+      float f[P::E];
+      kpow_factors<P>(a, term, iw, xq, t, f);
+#pragma unroll
+      for (int e = 0; e < P::E; ++e) v[e] = cscale(psi[e], f[e]);
     } else {
       col_factors<P, QM>(a, term, iw, xq, t, v);
 #pragma unroll

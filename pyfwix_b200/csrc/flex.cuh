@@ -710,8 +710,9 @@ __device__ __forceinline__ void col_factors(const SpecArgs& a, const Dim<S>& d, 
 #pragma unroll 1
     for (int r = 0; r < RT; ++r) q[r] = qmult<Q_PS_ADJ>(a, t, c.iw, c.x, c.j + r * d.nt());
   } else if (qm == Q_KPOW) {
+    const KPow k(a, t, c.iw, c.x);
 #pragma unroll
-    for (int r = 0; r < RT; ++r) q[r] = qmult<Q_KPOW>(a, t, c.iw, c.x, c.j + r * d.nt());
+    for (int r = 0; r < RT; ++r) q[r] = make_float2(k.at(c.j + r * d.nt()), 0.f);
   } else {
 #pragma unroll
     for (int r = 0; r < RT; ++r) q[r] = make_float2(a.norm, 0.f);

@@ -253,6 +253,32 @@ __device__ __forceinline__ float2 qmult(const SpecArgs& a, int t, int iw, int x,
   return QM == Q_PS_FWD ? make_float2(att * cs, -att * sn) : make_float2(att * cs, att * sn);
 }
 
+// Born filter (|k| / w)^(2n) x norm of term t (order n = t + term0) along a column
+// (fixed x): a real factor, k^2n by products and norm / w^2n once per column, so a
+// sample takes four instructions instead of two table loads, a division and a
+// complex product (the one-term column pass of the 256 x 256 x 128 scattering
+// adjoint was 68 us of a 20 us floor).  |ky| = |index| dk as in the wavenumber table.
+struct KPow {
+  float kx2, dk, s;
+  int n, NY;
+  __device__ __forceinline__ KPow(const SpecArgs& a, int t, int iw, int x) {
+    const float kx = a.kx[x];
+    kx2 = kx * kx;
+    dk = a.d.NY > 1 ? a.ky[1] : 0.f;
+    NY = a.d.NY;
+    n = t + a.term0;
+    s = a.norm;
+    for (int k = 0; k < n; ++k) s /= a.w2[iw];
+  }
+  __device__ __forceinline__ float at(int y) const {
+    const float ky = (float)min(y, NY - y) * dk;
+    const float k2 = kx2 + ky * ky;
+    float p = n == 0 ? 1.f : k2;
+    for (int k = 1; k < n; ++k) p *= k2;
+    return p * s;
+  }
+};
+
 // Phase-table view of one column (fixed x) for one term: the factors of every
 // ky of that column are then one load each (qcol_get).  Only for the cached
 // phase-shift path (a.ptab set, Q_PS_FWD / Q_PS_ADJ).

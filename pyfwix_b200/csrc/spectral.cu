@@ -458,31 +458,33 @@ cudaError_t launch_phase_shift(const SpecArgs& a, int mode, const float2* sref_w
 }
 
 // Forward phase factors x norm of one depth for every (ref, w, |kx|, |ky|): the
-// same arithmetic as the in-kernel evaluation (k depends on |index| only).
-__global__ void k_phase_table(const SpecArgs a, float2* dst) {
+// same arithmetic as the in-kernel evaluation (k depends on |index| only).  A CTA
+// takes kTableRows rows (of the slower of the two indices) of one (ref, w) slice, a
+// warp a row, so that a factor costs its root, exponential or sine, its table reads
+// and the store, and no index divisions.
+constexpr int kTableRows = 8;  // warps of a CTA
+__global__ void __launch_bounds__(256) k_phase_table(const SpecArgs a, int nblk, float2* dst) {
   chain_next();
   chain_wait();
-  const long long n = (long long)a.nterm * a.d.nw * a.ptab_nx * a.ptab_ny;
+  const bool ky_fast = a.ptab_sy == 1;
+  const int nf = ky_fast ? a.ptab_ny : a.ptab_nx, ns = ky_fast ? a.ptab_nx : a.ptab_ny;
+  const int slice = blockIdx.x / nblk, r = slice / a.d.nw, iw = slice - r * a.d.nw;
+  const int k0 = (blockIdx.x - slice * nblk) * kTableRows, rows = min(kTableRows, ns - k0);
   SpecArgs b = a;
   b.ptab = nullptr;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x) {
-    // the faster of the two indices first (a.ptab_sx, a.ptab_sy)
-    const int nf = a.ptab_sy == 1 ? a.ptab_ny : a.ptab_nx, ns = a.ptab_sy == 1 ? a.ptab_nx : a.ptab_ny;
-    const int kf = (int)(i % nf);
-    long long q = i / nf;
-    const int ks = (int)(q % ns);
-    q /= ns;
-    const int kxq = a.ptab_sy == 1 ? ks : kf, kyq = a.ptab_sy == 1 ? kf : ks;
-    const int iw = (int)(q % a.d.nw);
-    const int r = (int)(q / a.d.nw);
-    dst[i] = qmult<Q_PS_FWD>(b, r, iw, kxq, kyq);
-  }
+  dst += (long long)slice * nf * ns + (long long)k0 * nf;
+  const int ks = threadIdx.x / 32;  // a row per warp
+  if (ks >= rows) return;
+  dst += ks * nf;
+  for (int kf = threadIdx.x % 32; kf < nf; kf += 32)
+    dst[kf] = qmult<Q_PS_FWD>(b, r, iw, ky_fast ? k0 + ks : kf, ky_fast ? kf : k0 + ks);
 }
 
 cudaError_t launch_phase_table(const SpecArgs& a, float2* dst, cudaStream_t s) {
-  const long long n = (long long)a.nterm * a.d.nw * a.ptab_nx * a.ptab_ny;
-  const cudaError_t e = launch_chained(a.d.chained, k_phase_table, grid1d(n), 256, 0, s, a, dst);
+  const int ns = a.ptab_sy == 1 ? a.ptab_nx : a.ptab_ny;
+  const int nblk = (ns + kTableRows - 1) / kTableRows;
+  const cudaError_t e =
+      launch_chained(a.d.chained, k_phase_table, (unsigned)(nblk * a.nterm * a.d.nw), 256, 0, s, a, nblk, dst);
   if (e == cudaSuccess) count_launch();
   return e != cudaSuccess ? e : cudaGetLastError();
 }
