@@ -1,11 +1,13 @@
-// use the register-resident passes of fast.cuh; every other supported length uses
-// the per-warp Stockham passes of spectral.cu.  Rows dispatch on NX, columns on NY.
+// Rows dispatch on NX, columns on NY: compile-time plans (fast.cuh), run-time ones
+// (flex.cuh), and the per-warp Stockham passes of spectral.cu for the few lengths
+// that have neither.
 #include "flex.h"
 #include "internal.h"
 
-#define FWIX_FAST_DECL(TAG)                                                                            \
+#define FWIX_FAST_DECL_ROWS(TAG)                                                                       \
   cudaError_t row_forward_##TAG(const SpecArgs& a, int pre, cudaStream_t s);                           \
-  cudaError_t row_inverse_##TAG(const SpecArgs& a, int post, int pt, cudaStream_t s);                  \
+  cudaError_t row_inverse_##TAG(const SpecArgs& a, int post, int pt, cudaStream_t s);
+#define FWIX_FAST_DECL(TAG)                                                                            \
   cudaError_t col_type_a_##TAG(const SpecArgs& a, int q, cudaStream_t s);                              \
   cudaError_t col_type_b_##TAG(const SpecArgs& a, int q, cudaStream_t s);                              \
   cudaError_t col_fft_##TAG(const SpecArgs& a, int inv, const float2* in, float2* out, int add, float sc, \
@@ -23,6 +25,7 @@ FWIX_FAST_DECL(320)
 FWIX_FAST_DECL(384)
 FWIX_FAST_DECL(512)
 FWIX_FAST_DECL(640)
+FWIX_FAST_DECL_ROWS(256)
 }  // namespace fast
 
 bool fast_length(int n) {
@@ -45,34 +48,25 @@ bool fast_length(int n) {
 
 bool resident_length(int n) { return fast_length(n) || flex::has_plan(n); }
 
+// Rows run the compile-time plan (fast.cuh) at 256 only, one conflict-free exchange
+// in a warp's own shared memory: the Born pair at 256 x 256 x 128 takes 12.6 ms so and
+// 13.9 with flex.cuh's rows.  At the other planned lengths flex.cuh's split saves an
+// exchange (128 = 8 16 for 8 4 4, 320 = 16 20 for 20 4 4, 384 = 8 8 6 for 12 4 4 2) or its
+// CTAs of 128 threads hold more warps (64 = 8 8, 512 = 8 8 8); us per pass at 320 x 320 x
+// 80 with six references, compile-time against flex: inverse with labels 185 and 143,
+// forward with labels 148 and 101, plain forward 50 and 42; at 384 x 384 x 96 the
+// smooth step's 308 and 233, its adjoint's 252 and 198; the packed Born pair at
+// 512 x 512 x 64 27.9 and 26.7 ms.
 cudaError_t row_forward(const SpecArgs& a, int pre, cudaStream_t s) {
   switch (a.d.NX) {
-    case 64: return fast::row_forward_64(a, pre, s);
-    case 96: return fast::row_forward_96(a, pre, s);
-    case 128: return fast::row_forward_128(a, pre, s);
-    case 160: return fast::row_forward_160(a, pre, s);
-    case 192: return fast::row_forward_192(a, pre, s);
     case 256: return fast::row_forward_256(a, pre, s);
-    case 320: return fast::row_forward_320(a, pre, s);
-    case 384: return fast::row_forward_384(a, pre, s);
-    case 512: return fast::row_forward_512(a, pre, s);
-    case 640: return fast::row_forward_640(a, pre, s);
     default: return flex::has_plan(a.d.NX) ? flex::row_forward(a, pre, s) : generic_row_forward(a, pre, s);
   }
 }
 
 cudaError_t row_inverse(const SpecArgs& a, int post, int post_taper, cudaStream_t s) {
   switch (a.d.NX) {
-    case 64: return fast::row_inverse_64(a, post, post_taper, s);
-    case 96: return fast::row_inverse_96(a, post, post_taper, s);
-    case 128: return fast::row_inverse_128(a, post, post_taper, s);
-    case 160: return fast::row_inverse_160(a, post, post_taper, s);
-    case 192: return fast::row_inverse_192(a, post, post_taper, s);
     case 256: return fast::row_inverse_256(a, post, post_taper, s);
-    case 320: return fast::row_inverse_320(a, post, post_taper, s);
-    case 384: return fast::row_inverse_384(a, post, post_taper, s);
-    case 512: return fast::row_inverse_512(a, post, post_taper, s);
-    case 640: return fast::row_inverse_640(a, post, post_taper, s);
     default: return flex::has_plan(a.d.NX) ? flex::row_inverse(a, post, post_taper, s) : generic_row_inverse(a, post, post_taper, s);
   }
 }

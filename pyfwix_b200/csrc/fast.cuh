@@ -1560,10 +1560,10 @@ cudaError_t col_fft(const SpecArgs& a, int inverse, const float2* in, float2* ou
 }  // namespace fast
 }  // namespace fwix
 
-// One translation unit per line length instantiates the launchers of its plan
-// (FWIX_FAST_INSTANTIATE2: one plan for the row passes, another for the columns).
-#define FWIX_FAST_INSTANTIATE(PLAN, TAG) FWIX_FAST_INSTANTIATE2(PLAN, PLAN, TAG)
-#define FWIX_FAST_INSTANTIATE2(PLAN, CPLAN, TAG)                                                                   \
+// One translation unit per line length instantiates the launchers of its plan:
+// FWIX_FAST_ROWS and FWIX_FAST_COLS (rows and columns may use different plans;
+// lengths whose rows run flex.cuh instantiate only their columns).
+#define FWIX_FAST_ROWS(PLAN, TAG)                                                                           \
   namespace fwix {                                                                                          \
   namespace fast {                                                                                          \
   cudaError_t row_forward_##TAG(const SpecArgs& a, int pre, cudaStream_t s) {                               \
@@ -1572,6 +1572,11 @@ cudaError_t col_fft(const SpecArgs& a, int inverse, const float2* in, float2* ou
   cudaError_t row_inverse_##TAG(const SpecArgs& a, int post, int pt, cudaStream_t s) {                      \
     return row_inverse<PLAN>(a, post, pt, s);                                                               \
   }                                                                                                         \
+  }                                                                                                         \
+  }
+#define FWIX_FAST_COLS(CPLAN, TAG)                                                                          \
+  namespace fwix {                                                                                          \
+  namespace fast {                                                                                          \
   cudaError_t col_type_a_##TAG(const SpecArgs& a, int q, cudaStream_t s) { return col_type_a<CPLAN>(a, q, s); } \
   cudaError_t col_type_b_##TAG(const SpecArgs& a, int q, cudaStream_t s) { return col_type_b<CPLAN>(a, q, s); } \
   cudaError_t col_fft_##TAG(const SpecArgs& a, int inv, const float2* in, float2* out, int add, float sc,    \

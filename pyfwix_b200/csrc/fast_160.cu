@@ -1,4 +1,4 @@
-// Register-resident passes for lines of 160 samples: 8 lanes x 20 samples,
+// Register-resident column passes for lines of 160 samples: 8 lanes x 20 samples,
 // radix stages 20, 4, 2 (the radix-20 butterfly is a prime-factor 4 x 5
 // transform, so the first stage needs no twiddles and the line is exchanged
 // through shared memory once less than with radix-4 stages throughout).
@@ -8,4 +8,4 @@
 
 using FwixPlan160 = fwix::fast::Plan<160, 20, fwix::fast::Radices<20, 4, 2>, 0,
     fwix::fast::XSw<fwix::fast::xs(1, 1, 15), fwix::fast::xs(4, 7, 7), -1, fwix::fast::xs(2, 1, 7)>>;
-FWIX_FAST_INSTANTIATE(FwixPlan160, 160)
+FWIX_FAST_COLS(FwixPlan160, 160)

@@ -7,4 +7,5 @@
 
 using FwixRowPlan256 = fwix::fast::Plan<256, 16, fwix::fast::Radices<16, 16>, 1>;
 using FwixColPlan256 = fwix::fast::Plan<256, 16, fwix::fast::Radices<16, 16>, 0, fwix::fast::XSw<fwix::fast::xs(4, 1, 15), fwix::fast::xs(4, 1, 15)>>;
-FWIX_FAST_INSTANTIATE2(FwixRowPlan256, FwixColPlan256, 256)
+FWIX_FAST_ROWS(FwixRowPlan256, 256)
+FWIX_FAST_COLS(FwixColPlan256, 256)

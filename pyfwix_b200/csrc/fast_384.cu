@@ -1,4 +1,4 @@
-// Register-resident passes for lines of 384 samples: 32 lanes x 12 samples,
+// Register-resident column passes for lines of 384 samples: 32 lanes x 12 samples,
 // radix stages 12, 4, 4, 2 (the radix-12 butterfly is a prime-factor 4 x 3
 // transform, so the first stage needs no twiddles and the line is exchanged
 // through shared memory once less than with radix-4 stages throughout).
@@ -8,4 +8,4 @@
 
 using FwixPlan384 = fwix::fast::Plan<384, 12, fwix::fast::Radices<12, 4, 4, 2>, 0,
     fwix::fast::XSw<fwix::fast::xs(2, 1, 15), -1, -1, fwix::fast::xs(1, 1, 15), -1, fwix::fast::xs(2, 1, 15)>>;
-FWIX_FAST_INSTANTIATE(FwixPlan384, 384)
+FWIX_FAST_COLS(FwixPlan384, 384)

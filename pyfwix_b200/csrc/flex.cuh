@@ -121,14 +121,20 @@ struct Dim {
   }
 };
 
-// Resident CTAs that a Fixed line's registers are held to: enough for 512 to 768
-// threads per SM, by the largest radix (a radix's samples are 2 registers each,
-// and a pass holds two to three such sets).
+// Resident CTAs that a Fixed line's registers are held to.  `sets` counts what a
+// thread holds across a stage of the largest radix, in units of RT registers (a
+// complex set is 2, labels or hat indices 1); with that stage's samples and some
+// 30 registers of addresses and temporaries it bounds the threads an SM can hold.
 template <class S>
-constexpr int min_blocks(int threads, bool light = false, bool heavy = false) {
-  if (!S::kFixed) return 1;
-  const int want = light ? 1024 : heavy ? 512 : S::MAXR <= 10 ? 768 : S::MAXR <= 16 ? 640 : 512;
-  return want / threads < 1 ? 1 : want / threads;
+constexpr int min_blocks(int threads, int sets) {
+  if constexpr (!S::kFixed) {
+    return 1;
+  } else {
+    const int regs = (32 + sets * S::RT + 2 * S::MAXR + 7) / 8 * 8;
+    const int fit = 65536 / (regs * threads);
+    const int most = 1536 / threads;  // (more warps than that never paid)
+    return fit < 1 ? 1 : fit > most ? (most < 1 ? 1 : most) : fit;
+  }
 }
 
 // Calls f(std::integral_constant<int, R>) for the run-time radix R.
@@ -289,12 +295,16 @@ struct RowCtx {
 // Classes of row weights that share a kernel (the weight itself is a uniform
 // run-time switch within a class).
 enum RowClass { C_ONE, C_MASK, C_SCAT, C_SMOOTH, C_PAIR, C_DERIV };
+// What a row pass's thread holds across the terms (min_blocks).
+constexpr int row_sets(int cls) {
+  return cls == C_ONE ? 0 : cls == C_SCAT ? 2 : cls == C_PAIR || cls == C_DERIV ? 5 : 3;
+}
 
 // t1[term] = F_x(pre_term * in) for each term.  The row's samples are read once
 // into registers; a term whose weight vanishes on all of the CTA's rows (masks,
 // smooth weights) is written as zeros.
 template <class S, int CLS>
-__global__ void __launch_bounds__(S::ROW_THREADS, min_blocks<S>(S::ROW_THREADS, CLS == C_ONE))
+__global__ void __launch_bounds__(S::ROW_THREADS, min_blocks<S>(S::ROW_THREADS, row_sets(CLS)))
     k_row_fwd(const SpecArgs a, const __grid_constant__ Geo g, int pre) {
   constexpr int RT = S::RT;
   const Dim<S> d{g};
@@ -431,7 +441,7 @@ __global__ void __launch_bounds__(S::ROW_THREADS, min_blocks<S>(S::ROW_THREADS, 
 // out (+)= post * sum_term W_term * F_x^-1(t2[term]); terms that no sample of the
 // CTA's rows selects are skipped.
 template <class S, int CLS>
-__global__ void __launch_bounds__(S::ROW_THREADS, min_blocks<S>(S::ROW_THREADS, CLS == C_ONE, CLS == C_PAIR || CLS == C_DERIV))
+__global__ void __launch_bounds__(S::ROW_THREADS, min_blocks<S>(S::ROW_THREADS, row_sets(CLS)))
     k_row_inv(const SpecArgs a, const __grid_constant__ Geo g, int post, int post_taper) {
   constexpr int RT = S::RT;
   const Dim<S> d{g};
@@ -721,7 +731,7 @@ __device__ __forceinline__ void col_factors(const SpecArgs& a, const Dim<S>& d, 
 
 // t2[term] = F_y^-1(Q_term * F_y(t1[0])); the spectrum stays in registers.
 template <class S>
-__global__ void __launch_bounds__(S::COL_THREADS, min_blocks<S>(S::COL_THREADS))
+__global__ void __launch_bounds__(S::COL_THREADS, min_blocks<S>(S::COL_THREADS, 2))
     k_col_a(const SpecArgs a, const __grid_constant__ Geo g, int qm) {
   constexpr int RT = S::RT;
   const Dim<S> d{g};
@@ -771,7 +781,7 @@ __global__ void __launch_bounds__(S::COL_THREADS, min_blocks<S>(S::COL_THREADS))
 
 // t2[0] = F_y^-1(sum_term Q_term * F_y(t1[term])).
 template <class S>
-__global__ void __launch_bounds__(S::COL_THREADS, min_blocks<S>(S::COL_THREADS))
+__global__ void __launch_bounds__(S::COL_THREADS, min_blocks<S>(S::COL_THREADS, 2))
     k_col_b(const SpecArgs a, const __grid_constant__ Geo g, int qm) {
   constexpr int RT = S::RT;
   const Dim<S> d{g};
@@ -822,7 +832,7 @@ __global__ void __launch_bounds__(S::COL_THREADS, min_blocks<S>(S::COL_THREADS))
 
 // out (+)= scale * F_y^{-+1}(in): the column half of a plain 2D transform.
 template <class S, bool INV>
-__global__ void __launch_bounds__(S::COL_THREADS, min_blocks<S>(S::COL_THREADS))
+__global__ void __launch_bounds__(S::COL_THREADS, min_blocks<S>(S::COL_THREADS, 2))
     k_col_fft(const SpecArgs a, const __grid_constant__ Geo g, const float2* in, float2* out, int add, float scale) {
   constexpr int RT = S::RT;
   const Dim<S> d{g};

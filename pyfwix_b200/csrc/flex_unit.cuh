@@ -1,7 +1,12 @@
 // The host entry points of one compile-time radix FWIX_FLEX_RT (flex.cuh): the
 // lengths of FWIX_FLEX_FIXED, listed as X(ra, rb), run kernels compiled for their
-// radices, every other one the kernels with run-time radices.
+// radices, those of FWIX_FLEX_ROWS only their row passes (their columns have a
+// compile-time plan), every other one the kernels with run-time radices.
 #include "flex.cuh"
+
+#ifndef FWIX_FLEX_ROWS
+#define FWIX_FLEX_ROWS
+#endif
 
 #define FWIX_FLEX_JOIN2(a, b) a##b
 #define FWIX_FLEX_JOIN(a, b) FWIX_FLEX_JOIN2(a, b)
@@ -13,6 +18,7 @@ namespace flex {
   if (p.ra == ra_ && p.rb == rb_) return row_forward_s<Fixed<FWIX_FLEX_RT, ra_, rb_>>(a, p, pre, s);
 cudaError_t FWIX_FLEX_JOIN(row_forward_, FWIX_FLEX_RT)(const SpecArgs& a, const Line& p, int pre, cudaStream_t s) {
   FWIX_FLEX_FIXED
+  FWIX_FLEX_ROWS
   return row_forward_s<Run<FWIX_FLEX_RT>>(a, p, pre, s);
 }
 #undef X
@@ -21,6 +27,7 @@ cudaError_t FWIX_FLEX_JOIN(row_forward_, FWIX_FLEX_RT)(const SpecArgs& a, const 
 cudaError_t FWIX_FLEX_JOIN(row_inverse_, FWIX_FLEX_RT)(const SpecArgs& a, const Line& p, int post, int pt,
                                                        cudaStream_t s) {
   FWIX_FLEX_FIXED
+  FWIX_FLEX_ROWS
   return row_inverse_s<Run<FWIX_FLEX_RT>>(a, p, post, pt, s);
 }
 #undef X
