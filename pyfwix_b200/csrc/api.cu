@@ -140,8 +140,9 @@ struct fwix_plan {
   int pslots = 0;             // depth iz lives in slot iz % pslots
   std::vector<int> pslot_iz;  // depth whose current factors a slot holds, -1 for none
   int pq_nx() const { return d.NX / 2 + 1; }
-  // ky extent of the phase table rounded up to even: 16-byte rows for the TMA tiles
-  int pq_ny() const { return (d.NY / 2 + 2) & ~1; }
+  // ky extent of the phase table rounded up to even (16-byte rows for the TMA tiles),
+  // above 256 to a multiple of four (two boxes of a tile)
+  int pq_ny() const { return d.NY / 2 + 1 <= 256 ? (d.NY / 2 + 2) & ~1 : (d.NY / 2 + 4) & ~3; }
   long long pdepth() const { return (long long)desc.nref * d.nw * pq_nx() * pq_ny(); }
   float coef[5] = {1.f, 1.f / 2.f, 3.f / 8.f, 5.f / 16.f, 35.f / 128.f};  // Scatter.h:526
 

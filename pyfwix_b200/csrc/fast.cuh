@@ -172,6 +172,17 @@ __device__ __forceinline__ int pos_last(int t, int e) {  // output of the forwar
   return lpos<P, P::radix(P::NS - 1)>(t, e);
 }
 
+// min(y, N - y) of y = pos_last(t, e).  A lane's t < T, so that after unrolling all
+// elements but those whose T positions straddle N / 2 know their side: one addition
+// from a shared base instead of a minimum per element and term.
+template <class P>
+__device__ __forceinline__ int fold_last(int t, int e) {
+  const int c = pos_last<P>(0, e);
+  if (c + P::T - 1 <= P::N / 2) return t + c;
+  if (c >= P::N / 2) return P::N - c - t;
+  return min(t + c, P::N - c - t);
+}
+
 template <class P, bool REV, bool INV, int S>
 __device__ __forceinline__ void stages(float2 (&v)[P::E], int t, const float2* __restrict__ tw, float2* line) {
   using O = Order<P, REV>;
@@ -774,7 +785,7 @@ __device__ __forceinline__ void col_factors(const SpecArgs& a, int t, int iw, in
   if ((QM == Q_PS_FWD || QM == Q_PS_ADJ) && a.ptab) {
     const QCol qc = qcol<QM>(a, t, iw, x);
 #pragma unroll
-    for (int e = 0; e < P::E; ++e) q[e] = qcol_get(a, qc, pos_last<P>(lane_t, e));
+    for (int e = 0; e < P::E; ++e) q[e] = qcol_get(qc, fold_last<P>(lane_t, e));
   } else {
 #pragma unroll
     for (int e = 0; e < P::E; ++e) q[e] = qmult<QM>(a, t, iw, x, pos_last<P>(lane_t, e));
@@ -788,8 +799,7 @@ __device__ __forceinline__ void kpow_factors(const SpecArgs& a, int t, int iw, i
   if (k.n == 1) {  // the usual order, without the power loop
 #pragma unroll
     for (int e = 0; e < P::E; ++e) {
-      const int y = pos_last<P>(lane_t, e);
-      const float ky = (float)min(y, P::N - y) * k.dk;
+      const float ky = (float)fold_last<P>(lane_t, e) * k.dk;
       f[e] = (k.kx2 + ky * ky) * k.s;
     }
   } else {
@@ -939,12 +949,32 @@ struct ColTma {
   static constexpr int NBOX = P::N <= 256 ? 1 : (P::N % 2 == 0 && P::N / 2 <= 256 ? 2 : 4);
   static constexpr int ROWS = P::N / NBOX;  // rows per box (<= 256)
   static_assert(ROWS * NBOX == P::N && ROWS <= 256, "a tile is a whole number of boxes of at most 256 rows");
-  // two tiles, the twiddles, two mbarriers, and room to align the tiles to 1024
-  // bytes; with the phase tiles (qt samples each: LX |kx| rows of the cached
-  // quarter spectrum) two of those after the term tiles
-  static size_t smem(size_t qt = 0) {
-    return (size_t)(2 * TILE + 2 * qt) * sizeof(float2) + tw_size<P>() * sizeof(float2) + 16 + 1024;
+  // two tiles, the phase tiles (qt samples each: LX |kx| rows of the cached quarter
+  // spectrum; none without them), the twiddles, up to four mbarriers, and room to align the
+  // tiles to 1024 bytes
+  __host__ __device__ static constexpr size_t smem_slots(size_t qt, int slots) {
+    return (size_t)(2 * TILE + slots * qt) * sizeof(float2) + tw_size<P>() * sizeof(float2) + 32 + 1024;
   }
+  // a phase tile comes in one box, or in two of half its ky (a box holds 256): ky
+  // extent of a table row, of a box
+  static constexpr int QBOX = P::N / 2 + 1 <= 256 ? 1 : 2;
+  static constexpr int PNY = QBOX == 1 ? (P::N / 2 + 2) & ~1 : (P::N / 2 + 4) & ~3;
+  static constexpr int QROWS = PNY / QBOX;
+  static constexpr size_t QT = (size_t)LX * PNY;
+  // sample ky of row `row` (times QROWS) of a phase tile
+  __device__ static __forceinline__ int qat(int row, int ky) {
+    return QBOX == 1 || ky < QROWS ? row + ky : row + LX * QROWS + ky - QROWS;
+  }
+  __host__ __device__ static constexpr int fit(int slots) {
+    return (int)((227 * 1024) / (smem_slots(QT, slots) + 1024));
+  }
+  // Phase tiles held at once: two (each term's fetched two terms ahead) where that
+  // leaves room for two CTAs per SM, else one, fetched once the term before has
+  // read its own (320 x 320 x 80: one CTA and two slots 244 and 227 us for the
+  // multi- and single-input pass, two CTAs and one slot 202 and 216; 256, where two
+  // CTAs fit either way: 127 us single-input with two slots, 135 with one).
+  static constexpr int SLOTS = fit(2) >= 2 ? 2 : 1;
+  __host__ __device__ static constexpr size_t smem(size_t qt = 0) { return smem_slots(qt, SLOTS); }
 };
 
 // The CTA's columns x0 .. x0 + LX - 1 read the phase factors of |kx| = min(x, NX - x):
@@ -967,11 +997,23 @@ __device__ __forceinline__ bool qflip(const SpecArgs& a, int t, int iw) {
   return !(a.w2[iw] * (sr.y - a.eps * sr.x) > 0.f);
 }
 
-// kQT: the phase factors of each term come as a TMA tile with the term's column
-// tile (the cached table of the phase shift modes); else col_factors loads them
-// from global memory before the tile wait.
+// Resident CTAs a TMA column pass is held to: what its shared memory lets an SM hold,
+// as far as its registers go: two for 12 samples per lane and more (three for the
+// single-input pass of 16 without phase tiles; 12 at three spilled 180 - 260 bytes in
+// the multi-input pass, 314 -> 339 us at 384 x 384 x 96), four for 8.
+template <class P>
+constexpr int col_tma_min_blocks(bool qtile, bool single) {
+  const int fit = qtile ? ColTma<P>::fit(ColTma<P>::SLOTS)
+                        : (int)((227 * 1024) / (ColTma<P>::smem_slots(0, 0) + 1024));
+  const int regs = P::E <= 8 ? 4 : P::E == 16 ? (single && !qtile ? FWIX_COLA_MINB16 : FWIX_COLB_MINB16) : 2;
+  return fit < 1 ? 1 : fit < regs ? fit : regs;
+}
+
+// kQT: the phase factors of each term come as a TMA tile (the cached table of the
+// phase shift modes); else col_factors loads them from global memory before the
+// tile wait.
 template <class P, int QM, bool kQT>
-__global__ void __launch_bounds__(kWarps * 32, ColGeo<P>::kMinBlocks)
+__global__ void __launch_bounds__(kWarps * 32, col_tma_min_blocks<P>(kQT, false))
     k_col_b_tma(const SpecArgs a, int nxt, const __grid_constant__ CUtensorMap tin,
                 const __grid_constant__ CUtensorMap tout, const __grid_constant__ CUtensorMap tq) {
   using C = ColTma<P>;
@@ -979,11 +1021,10 @@ __global__ void __launch_bounds__(kWarps * 32, ColGeo<P>::kMinBlocks)
   extern __shared__ unsigned char smem_raw[];
   float2* base = reinterpret_cast<float2*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   float2* tiles[2] = {base, base + C::TILE};
-  const int pny = a.ptab_ny;
-  const int qt = kQT ? C::LX * pny : 0;  // samples per phase tile (pny even: 128-byte multiples)
-  float2* qs[2] = {base + 2 * C::TILE, base + 2 * C::TILE + qt};
-  float2* tw = base + 2 * C::TILE + 2 * qt;
-  uint64_t* bar = reinterpret_cast<uint64_t*>(tw + tw_size<P>());
+  constexpr int qt = kQT ? (int)C::QT : 0;  // samples of a phase tile (a multiple of 128 bytes)
+  float2* const qs = base + 2 * C::TILE;
+  float2* tw = base + 2 * C::TILE + C::SLOTS * qt;
+  uint64_t* bar = reinterpret_cast<uint64_t*>(tw + tw_size<P>());  // tiles 0 and 1, a phase tile of its own
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane / P::T, t = lane % P::T, col = warp * P::G + g;
   const long long b = blockIdx.x / nxt;  // launch-local slice
@@ -993,39 +1034,62 @@ __global__ void __launch_bounds__(kWarps * 32, ColGeo<P>::kMinBlocks)
   const int xq = x < a.d.NX ? x : 0;
   const int zstride = (int)(a.tstride / a.d.slice);  // slices per term in t1
   const int k0 = qtile_k0<P>(a, x0);
-  const int qrow = qtile_row(a, xq, k0, C::LX) * pny;
+  const int qrow = qtile_row(a, xq, k0, C::LX) * C::QROWS;
   if (threadIdx.x == 0) {
     tma::mbar_init(&bar[0], 1);
     tma::mbar_init(&bar[1], 1);
+    tma::mbar_init(&bar[2], 1);
     tma::fence_mbar_init();
   }
   chain_next();
   load_stage_tw<P>(tw, a.twy);
   chain_wait();
   __syncthreads();
+  // The phase tile of `term`: with two slots beside the term's tile, on its barrier;
+  // with one slot on a barrier of its own, once the term before has read it.
+  constexpr bool kOwn = kQT && C::SLOTS == 1;
+  auto load_q = [&](int term, int slot, uint64_t* qb) {
+#pragma unroll
+    for (int h = 0; h < C::QBOX; ++h)
+      tma::load_3d(qs + slot * qt + h * C::LX * C::QROWS, &tq, h * C::QROWS, k0, term * a.d.nw + iw, qb);
+  };
   auto issue = [&](int term, int buf) {
-    tma::mbar_expect_tx(&bar[buf], (unsigned)((C::TILE + qt) * sizeof(float2)));
+    tma::mbar_expect_tx(&bar[buf], (unsigned)((C::TILE + (kOwn ? 0 : qt)) * sizeof(float2)));
 #pragma unroll
     for (int k = 0; k < C::NBOX; ++k)
       tma::load_3d(tiles[buf] + k * C::ROWS * C::LX, &tin, x0, k * C::ROWS, term * zstride + (int)b, &bar[buf]);
-    if constexpr (kQT) tma::load_3d(qs[buf], &tq, 0, k0, term * a.d.nw + iw, &bar[buf]);
+    if constexpr (kQT && !kOwn) load_q(term, buf, &bar[buf]);
   };
-  if (threadIdx.x == 0) issue(0, 0);
+  auto issue_q = [&](int term) {
+    if (term >= a.nterm) return;
+    tma::mbar_expect_tx(&bar[2], (unsigned)(qt * sizeof(float2)));
+    load_q(term, 0, &bar[2]);
+  };
+  if (threadIdx.x == 0) {
+    issue(0, 0);
+    if constexpr (kOwn) issue_q(0);
+  }
+  // Bounded-wait failure: count it and let the loads in flight land (bounded): the
+  // next tile and, on its own barrier, the phase tile.
+  auto bail = [&](int term) {
+    if (threadIdx.x != 0) return;
+    atomicAdd(a.err, 1u);
+    if (term + 1 < a.nterm) tma::mbar_wait(&bar[(term + 1) & 1], (unsigned)((term + 1) >> 1) & 1u);
+    if constexpr (kOwn) tma::mbar_wait(&bar[2], (unsigned)term & 1u);
+  };
   float2 acc[P::E];
 #pragma unroll
   for (int e = 0; e < P::E; ++e) acc[e] = make_float2(0.f, 0.f);
+  bool good = true;  // no wait of this thread has run out (checked with the next barrier that can)
   for (int term = 0; term < a.nterm; ++term) {
     const int buf = term & 1;
     if (threadIdx.x == 0 && term + 1 < a.nterm) issue(term + 1, buf ^ 1);
     constexpr bool kQ = !kQT && QM != Q_KPOW;
     float2 q[kQ ? P::E : 1];
     if constexpr (kQ) col_factors<P, QM>(a, term, iw, xq, t, q);
-    const bool ok = tma::mbar_wait(&bar[buf], (unsigned)(term >> 1) & 1u);
-    if (!__syncthreads_and(ok)) {
-      if (threadIdx.x == 0) {
-        atomicAdd(a.err, 1u);
-        if (term + 1 < a.nterm) tma::mbar_wait(&bar[buf ^ 1], (unsigned)((term + 1) >> 1) & 1u);
-      }
+    good = tma::mbar_wait(&bar[buf], (unsigned)(term >> 1) & 1u) && good;
+    if (!__syncthreads_and(good)) {
+      bail(term);
       return;
     }
     float2 v[P::E];
@@ -1034,12 +1098,12 @@ __global__ void __launch_bounds__(kWarps * 32, ColGeo<P>::kMinBlocks)
     __syncthreads();  // the tile is in registers: its buffer is free for the exchanges
     fft_fwd<P>(v, t, tw, tiles[buf] + col * P::N);
     if constexpr (kQT) {
-      const float2* qr = qs[buf] + qrow;
+      if constexpr (kOwn) good = tma::mbar_wait(&bar[2], (unsigned)term & 1u);
+      const float2* qr = qs + (kOwn ? 0 : buf) * qt;
       const bool flip = qflip<QM>(a, term, iw);
 #pragma unroll
       for (int e = 0; e < P::E; ++e) {
-        const int ky = pos_last<P>(t, e);
-        const float2 f = qr[min(ky, P::N - ky)];
+        const float2 f = qr[C::qat(qrow, fold_last<P>(t, e))];
         acc[e] = cadd(acc[e], cmul(v[e], flip ? cconj(f) : f));
       }
     } else if constexpr (QM == Q_KPOW) {
@@ -1051,15 +1115,25 @@ __global__ void __launch_bounds__(kWarps * 32, ColGeo<P>::kMinBlocks)
 #pragma unroll
       for (int e = 0; e < P::E; ++e) acc[e] = cadd(acc[e], cmul(v[e], q[e]));
     }
-    tma::fence_proxy_async();  // the exchanges and phase reads precede the next loads into this buffer
+    tma::fence_proxy_async();  // the exchanges and phase reads precede the next loads into their places
     __syncthreads();
+    if constexpr (kOwn) {
+      if (threadIdx.x == 0) issue_q(term + 1);
+    }
   }
   // no load is pending: buffer 0 holds the inverse transform's exchanges, buffer 1 the result
   fft_inv<P>(acc, t, tw, tiles[0] + col * P::N);
 #pragma unroll
   for (int e = 0; e < P::E; ++e) tiles[1][tma::swz_tile<C::LX>(pos_first<P>(t, e), col)] = acc[e];
   tma::fence_proxy_async();
-  __syncthreads();
+  if constexpr (kOwn) {
+    if (!__syncthreads_and(good)) {
+      if (threadIdx.x == 0) atomicAdd(a.err, 1u);
+      return;
+    }
+  } else {
+    __syncthreads();
+  }
   if (threadIdx.x == 0) {
 #pragma unroll
     for (int k = 0; k < C::NBOX; ++k) tma::store_3d(&tout, x0, k * C::ROWS, (int)b, tiles[1] + k * C::ROWS * C::LX);
@@ -1077,27 +1151,14 @@ __global__ void __launch_bounds__(kWarps * 32, ColGeo<P>::kMinBlocks)
 template <class P>
 struct ColTmaA {
   static constexpr int LX = ColTma<P>::LX, TILE = ColTma<P>::TILE, NBOX = ColTma<P>::NBOX, ROWS = ColTma<P>::ROWS;
-  // input tile (then the exchange lines), staging tile, two phase tiles of qt
-  // samples (none without them), twiddles, three mbarriers, alignment room
-  static size_t smem(size_t qt = 0) {
-    return (size_t)(2 * TILE + 2 * qt) * sizeof(float2) + tw_size<P>() * sizeof(float2) + 24 + 1024;
-  }
+  static constexpr int SLOTS = ColTma<P>::SLOTS;
+  // input tile (then the exchange lines), staging tile, the phase tiles of qt samples
+  // (none without them), twiddles, mbarriers, alignment room
+  static constexpr size_t smem(size_t qt = 0) { return ColTma<P>::smem(qt); }
 };
 
-// Resident CTAs the single-input TMA pass is held to: with the phase tiles its
-// shared memory (two tiles, two phase tiles) leaves room for fewer CTAs than the
-// register budget of ColGeo::kMinBlocksA would allow, and registers beyond that
-// budget only avoid spills.
-template <class P>
-constexpr int col_a_tma_min_blocks(bool qtile) {
-  constexpr int LX = ColGeo<P>::LX;
-  constexpr size_t per = (size_t)(2 * P::N * LX + 2 * LX * ((P::N / 2 + 2) & ~1) + tw_size<P>()) * 8 + 24 + 1024;
-  constexpr int fit = (int)((227 * 1024) / per) > 0 ? (int)((227 * 1024) / per) : 1;
-  return qtile && fit < ColGeo<P>::kMinBlocksA ? fit : ColGeo<P>::kMinBlocksA;
-}
-
 template <class P, int QM, bool kQT>
-__global__ void __launch_bounds__(kWarps * 32, col_a_tma_min_blocks<P>(kQT))
+__global__ void __launch_bounds__(kWarps * 32, col_tma_min_blocks<P>(kQT, true))
     k_col_a_tma(const SpecArgs a, int nxt, const __grid_constant__ CUtensorMap tin,
                 const __grid_constant__ CUtensorMap tout, const __grid_constant__ CUtensorMap tq) {
   using C = ColTmaA<P>;
@@ -1105,11 +1166,11 @@ __global__ void __launch_bounds__(kWarps * 32, col_a_tma_min_blocks<P>(kQT))
   extern __shared__ unsigned char smem_raw[];
   float2* in = reinterpret_cast<float2*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   float2* stage = in + C::TILE;
-  const int pny = a.ptab_ny;
-  const int qt = kQT ? C::LX * pny : 0;
-  float2* const q0 = stage + C::TILE;  // phase slot k at q0 + k * qt
-  float2* tw = stage + C::TILE + 2 * qt;
-  uint64_t* bar = reinterpret_cast<uint64_t*>(tw + tw_size<P>());  // input, phase slot 0, phase slot 1
+  using T = ColTma<P>;
+  constexpr int qt = kQT ? (int)T::QT : 0;
+  float2* const qs = stage + C::TILE;
+  float2* tw = stage + C::TILE + C::SLOTS * qt;
+  uint64_t* bar = reinterpret_cast<uint64_t*>(tw + tw_size<P>());  // input, phase tiles
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane / P::T, t = lane % P::T, col = warp * P::G + g;
   const long long b = blockIdx.x / nxt;
@@ -1119,49 +1180,47 @@ __global__ void __launch_bounds__(kWarps * 32, col_a_tma_min_blocks<P>(kQT))
   const int xq = x < a.d.NX ? x : 0;
   const int zstride = (int)(a.tstride / a.d.slice);
   const int k0 = qtile_k0<P>(a, x0);
-  const int qrow = qtile_row(a, xq, k0, C::LX) * pny;
+  const int qrow = qtile_row(a, xq, k0, C::LX) * T::QROWS;
   const int nterm = a.nterm;
   if (threadIdx.x == 0) {
-    tma::mbar_init(&bar[0], 1);
-    tma::mbar_init(&bar[1], 1);
-    tma::mbar_init(&bar[2], 1);
+    for (int k = 0; k < 1 + C::SLOTS; ++k) tma::mbar_init(&bar[k], 1);
     tma::fence_mbar_init();
   }
   chain_next();
   load_stage_tw<P>(tw, a.twy);
   chain_wait();
   __syncthreads();
-  auto issue_q = [&](int term) {  // the phase tile of `term` into slot term & 1
-    uint64_t* qb = &bar[1 + (term & 1)];
-    tma::mbar_expect_tx(qb, (unsigned)(qt * sizeof(float2)));
-    tma::load_3d(q0 + (term & 1) * qt, &tq, 0, k0, term * a.d.nw + iw, qb);
+  auto issue_q = [&](int term) {  // the phase tile of `term` into slot term mod SLOTS (1 or 2)
+    if (term >= nterm) return;
+    const int k = term & (C::SLOTS - 1);
+    tma::mbar_expect_tx(&bar[1 + k], (unsigned)(qt * sizeof(float2)));
+#pragma unroll
+    for (int h = 0; h < T::QBOX; ++h)
+      tma::load_3d(qs + k * qt + h * C::LX * T::QROWS, &tq, h * T::QROWS, k0, term * a.d.nw + iw, &bar[1 + k]);
+  };
+  auto wait_q = [&](int term) {
+    return tma::mbar_wait(&bar[1 + (term & (C::SLOTS - 1))], (unsigned)(term >> (C::SLOTS - 1)) & 1u);
   };
   if (threadIdx.x == 0) {
     tma::mbar_expect_tx(&bar[0], (unsigned)(C::TILE * sizeof(float2)));
 #pragma unroll
     for (int k = 0; k < C::NBOX; ++k) tma::load_3d(in + k * C::ROWS * C::LX, &tin, x0, k * C::ROWS, (int)b, &bar[0]);
-    if constexpr (kQT) {
-      if (nterm > 0) issue_q(0);
-      if (nterm > 1) issue_q(1);
-    }
+    if constexpr (kQT)
+      for (int k = 0; k < C::SLOTS; ++k) issue_q(k);
   }
-  // Bounded-wait failure: count it, let the loads in flight land (bounded) and
-  // the committed stores read their source, then leave together.
-  auto bail = [&](int pending_q) {
-    if (threadIdx.x == 0) {
-      atomicAdd(a.err, 1u);
-      if (kQT && pending_q >= 0 && pending_q < nterm)
-        tma::mbar_wait(&bar[1 + (pending_q & 1)], (unsigned)(pending_q >> 1) & 1u);
-      tma::store_wait_read();
-    }
+  // Bounded-wait failure: count it, let the phase loads in flight (terms q to
+  // before `end`) land (bounded) and the committed stores read their source, then
+  // leave together.
+  auto bail = [&](int q, int end) {
+    if (threadIdx.x != 0) return;
+    atomicAdd(a.err, 1u);
+    if constexpr (kQT)
+      for (; q < end && q < nterm; ++q) wait_q(q);
+    tma::store_wait_read();
   };
   const bool ok = tma::mbar_wait(&bar[0], 0u);
   if (!__syncthreads_and(ok)) {
-    if (threadIdx.x == 0 && kQT) {
-      // the phase loads of terms 0 and 1 may be in flight
-      for (int k = 0; k < 2 && k < nterm; ++k) tma::mbar_wait(&bar[1 + k], 0u);
-    }
-    bail(-1);
+    bail(0, C::SLOTS);
     return;
   }
   float2 psi[P::E];
@@ -1197,17 +1256,16 @@ __global__ void __launch_bounds__(kWarps * 32, col_a_tma_min_blocks<P>(kQT))
   for (int term = first; term < nterm; ++term) {
     float2 v[P::E];
     if constexpr (kQT) {
-      const bool qok = tma::mbar_wait(&bar[1 + (term & 1)], (unsigned)(term >> 1) & 1u);
+      const bool qok = wait_q(term);
       if (!__syncthreads_and(qok)) {
-        bail(term + 1);
+        bail(term + 1, term + C::SLOTS);
         return;
       }
-      const float2* qr = q0 + (term & 1) * qt + qrow;
+      const float2* qr = qs + (term & (C::SLOTS - 1)) * qt;
       const bool flip = qflip<QM>(a, term, iw);
 #pragma unroll
       for (int e = 0; e < P::E; ++e) {
-        const int ky = pos_last<P>(t, e);
-        const float2 f = qr[min(ky, P::N - ky)];
+        const float2 f = qr[T::qat(qrow, fold_last<P>(t, e))];
         v[e] = cmul(psi[e], flip ? cconj(f) : f);
       }
     } else if constexpr (QM == Q_KPOW) {
@@ -1222,12 +1280,12 @@ __global__ void __launch_bounds__(kWarps * 32, col_a_tma_min_blocks<P>(kQT))
     }
     fft_inv<P>(v, t, tw, line);
     stage_free();
+    if constexpr (kQT) {  // every lane has read this term's factors
+      if (threadIdx.x == 0) issue_q(term + C::SLOTS);
+    }
 #pragma unroll
     for (int e = 0; e < P::E; ++e) stage[tma::swz_tile<C::LX>(pos_first<P>(t, e), col)] = v[e];
-    store(term);  // also orders this term's phase reads before the slot's next load
-    if constexpr (kQT) {
-      if (threadIdx.x == 0 && term + 2 < nterm) issue_q(term + 2);
-    }
+    store(term);
   }
   if (threadIdx.x == 0) tma::store_wait_read();
 }
@@ -1395,14 +1453,14 @@ cudaError_t row_inverse(const SpecArgs& a, int post, int post_taper, cudaStream_
 
 // Whether a TMA column pass of plan P takes its phase factors as TMA tiles: the
 // phase-shift modes with the cached table, asked for in a.qtile (bit 0 the
-// multi-input pass k_col_b, bit 1 the single-input k_col_a), rows of at most 256
-// even-length entries, and tiles that never straddle NX / 2 (so that a tile's |kx|
-// are consecutive).
+// multi-input pass k_col_b, bit 1 the single-input k_col_a), the table's rows as the
+// tile expects them, and tiles that never straddle NX / 2 (so that a tile's |kx| are
+// consecutive).
 template <class P>
 bool use_qtile(const SpecArgs& a, int qmode, int bit) {
   constexpr int LX = ColGeo<P>::LX;
-  return ((a.qtile >> bit) & 1) && (qmode == Q_PS_FWD || qmode == Q_PS_ADJ) && a.ptab && a.ptab_ny % 2 == 0 &&
-         a.ptab_ny <= 256 && (a.d.NX / 2) % LX == 0 && a.ptab_nx >= LX;
+  return ((a.qtile >> bit) & 1) && (qmode == Q_PS_FWD || qmode == Q_PS_ADJ) && a.ptab &&
+         a.ptab_ny == ColTma<P>::PNY && a.ptab_sy == 1 && (a.d.NX / 2) % LX == 0 && a.ptab_nx >= LX;
 }
 
 template <class P>
@@ -1411,12 +1469,12 @@ cudaError_t col_type_a_tma(const SpecArgs& a, int qmode, cudaStream_t s) {
   const int nxt = (a.d.NX + C::LX - 1) / C::LX;
   const unsigned grid = (unsigned)(a.nb * nxt);
   const bool qtile = use_qtile<P>(a, qmode, 1);
-  const size_t sm = C::smem(qtile ? (size_t)C::LX * a.ptab_ny : 0);
+  const size_t sm = C::smem(qtile ? ColTma<P>::QT : 0);
   CUtensorMap tin, tout, tq;
   std::memset(&tq, 0, sizeof(tq));
   cudaError_t e = tile_map(&tin, a.t1, a.d.NX, a.d.NY, a.nb, C::ROWS, C::LX);
   if (e == cudaSuccess) e = tile_map(&tout, a.t2, a.d.NX, a.d.NY, (a.tstride / a.d.slice) * (a.term0 + a.nterm), C::ROWS, C::LX);
-  if (e == cudaSuccess && qtile) e = qtab_map(&tq, a.ptab, a.ptab_ny, a.ptab_nx, (long long)a.nterm * a.d.nw, C::LX);
+  if (e == cudaSuccess && qtile) e = qtab_map(&tq, a.ptab, a.ptab_ny, a.ptab_nx, (long long)a.nterm * a.d.nw, C::LX, ColTma<P>::QROWS);
   if (e != cudaSuccess) return e;
 #define FWIX_FAST_CAT(Q, QT)                                                                          \
   e = opt_in_smem(k_col_a_tma<P, Q, QT>, sm);                                                         \
@@ -1479,12 +1537,12 @@ cudaError_t col_type_b_tma(const SpecArgs& a, int qmode, cudaStream_t s) {
   const int nxt = (a.d.NX + C::LX - 1) / C::LX;
   const unsigned grid = (unsigned)(a.nb * nxt);
   const bool qtile = use_qtile<P>(a, qmode, 0);
-  const size_t sm = C::smem(qtile ? (size_t)C::LX * a.ptab_ny : 0);
+  const size_t sm = C::smem(qtile ? ColTma<P>::QT : 0);
   CUtensorMap tin, tout, tq;
   std::memset(&tq, 0, sizeof(tq));
   cudaError_t e = tile_map(&tin, a.t1, a.d.NX, a.d.NY, (a.tstride / a.d.slice) * a.nterm, C::ROWS, C::LX);
   if (e == cudaSuccess) e = tile_map(&tout, a.t2, a.d.NX, a.d.NY, a.nb, C::ROWS, C::LX);
-  if (e == cudaSuccess && qtile) e = qtab_map(&tq, a.ptab, a.ptab_ny, a.ptab_nx, (long long)a.nterm * a.d.nw, C::LX);
+  if (e == cudaSuccess && qtile) e = qtab_map(&tq, a.ptab, a.ptab_ny, a.ptab_nx, (long long)a.nterm * a.d.nw, C::LX, ColTma<P>::QROWS);
   if (e != cudaSuccess) return e;
 #define FWIX_FAST_CBT(Q, QT)                                                                          \
   e = opt_in_smem(k_col_b_tma<P, Q, QT>, sm);                                                         \

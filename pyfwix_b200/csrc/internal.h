@@ -83,7 +83,7 @@ struct SpecArgs {
   // cached forward phase factors of this depth (x norm), element (ref, iw, |kx|, |ky|)
   // at ptab[(ref*nw + iw)*ptab_nx*ptab_ny + kxq*ptab_sx + kyq*ptab_sy], kxq =
   // min(x, NX-x), kyq = min(y, NY-y); ptab_nx = NX/2 + 1, ptab_ny = NY/2 + 1 rounded
-  // up to even (16-byte rows for TMA).  ky runs fastest for the columns whose lanes
+  // up to even, above 256 to a multiple of four (16-byte rows and boxes for TMA).  ky runs fastest for the columns whose lanes
   // run along ky (compile-time plans), kx for those whose lanes run across the
   // columns (flex.cuh).  NULL means evaluate the factors in the kernel
   const float2* ptab;

@@ -299,8 +299,9 @@ __device__ __forceinline__ QCol qcol(const SpecArgs& a, int t, int iw, int x) {
   }
   return q;
 }
-__device__ __forceinline__ float2 qcol_get(const SpecArgs& a, const QCol& q, int y) {
-  const float2 P = q.p[min(y, a.d.NY - y)];
+// The factor at folded row ky = min(y, NY - y).
+__device__ __forceinline__ float2 qcol_get(const QCol& q, int ky) {
+  const float2 P = q.p[ky];
   return q.flip ? cconj(P) : P;
 }
 

@@ -101,8 +101,9 @@ cudaError_t tile_map(CUtensorMap* out, const void* base, int nx, int ny, long lo
 
 // Host side: a 3-D tensor map over the quarter-spectrum phase table of one depth,
 // [nslices][pnx][pny] 8-byte factors (ky fastest, pny even so that rows are 16-byte
-// multiples), box {pny, box_cols, 1} (every ky of box_cols consecutive kx of one
-// (reference, frequency) slice), no swizzle.  Cached like tile_map.
-cudaError_t qtab_map(CUtensorMap* out, const void* base, int pny, int pnx, long long nslices, int box_cols);
+// multiples), box {box_rows, box_cols, 1} (box_rows ky, even, of box_cols consecutive
+// kx of one (reference, frequency) slice), no swizzle.  Cached like tile_map.
+cudaError_t qtab_map(CUtensorMap* out, const void* base, int pny, int pnx, long long nslices, int box_cols,
+                     int box_rows);
 
 }  // namespace fwix
