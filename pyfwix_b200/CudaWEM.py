@@ -118,6 +118,19 @@ def _dev(x, device, shape=None, zero=False):
     return t.to(device=device, dtype=torch.complex64).contiguous()
 
 
+def _out(x, device, src):
+    """Device tensor for a result that the operator writes in full, computed from the
+    device tensor ``src``: the operand itself where it is one, without the zero fill
+    of a sum (a launch and a pass over the field).  An operand that shares its memory
+    with ``src``, or is not of its size, is zeroed first, as a sum's would be."""
+    t = _raw(x)
+    if (isinstance(t, torch.Tensor) and t.device == device and t.dtype == torch.complex64 and t.is_contiguous()
+            and t.numel() == src.numel()
+            and t.untyped_storage().data_ptr() != src.untyped_storage().data_ptr()):
+        return t
+    return _dev(x, device, zero=True)
+
+
 def _store(dst, t):
     """Copy a device result back into the caller's object when it is not the
     same memory."""
@@ -476,16 +489,18 @@ class _OneStep:
 
     def forward(self, add, model, data):
         with torch.cuda.device(self.device):
-            out = _dev(data, self.device) if add else _dev(data, self.device, zero=True)
-            self.plan.step(self.iz, _dev(model, self.device), out, direction=L.FWD, add=bool(add))
+            m = _dev(model, self.device)
+            out = _dev(data, self.device) if add else _out(data, self.device, m)
+            self.plan.step(self.iz, m, out, direction=L.FWD, add=bool(add))
             _store(data, out)
 
     def adjoint(self, add, model, data):
         """Add-version adjoint: for PSPI it leaves out the taper, as the
         reference's ``PSPI::cu_adjoint(bool, ...)`` does (``propagator/src/PSPI.cpp:26-44``)."""
         with torch.cuda.device(self.device):
-            out = _dev(model, self.device) if add else _dev(model, self.device, zero=True)
-            self.plan.step(self.iz, _dev(data, self.device), out, direction=L.ADJ_ADD, add=bool(add))
+            d = _dev(data, self.device)
+            out = _dev(model, self.device) if add else _out(model, self.device, d)
+            self.plan.step(self.iz, d, out, direction=L.ADJ_ADD, add=bool(add))
             _store(model, out)
 
 

@@ -109,7 +109,8 @@ class Plan:
         if labels.dim() != 4 or tuple(labels.shape[2:]) != (self.NY, self.NX) or labels.shape[0] != self.nz \
                 or labels.shape[1] not in (1, self.nw):
             raise ValueError(f"labels shape {tuple(labels.shape)} does not match [nz][nw|1][NY][NX]")
-        if labels.numel() and (int(labels.min()) < 0 or int(labels.max()) > 255):
+        # (bytes cannot lie outside; asking would wait for the device)
+        if labels.dtype != torch.uint8 and labels.numel() and (int(labels.min()) < 0 or int(labels.max()) > 255):
             raise ValueError("labels must lie in [0, 255]")
         labels = labels.to(device=self.device, dtype=torch.uint8).contiguous()
         wst = 0 if labels.shape[1] == 1 else self.NY * self.NX
