@@ -372,7 +372,7 @@ template <class P, int PRE, bool RF = false>
 __global__ void __launch_bounds__(kWarps * 32, row_fwd_min_blocks<P, PRE>()) k_row_fwd(const SpecArgs a, int nchunk) {
   extern __shared__ float2 smem[];
   RowCtx<P> c(a, smem, nchunk);
-  chain_next();
+  if (a.early) chain_next();
   load_stage_tw<P>(c.tw, a.twx);
   chain_wait();
   prefetch_next_ctas<P::N, RowGeo<P>::ROWS>(a, a.in, false, nchunk);
@@ -497,6 +497,7 @@ __global__ void __launch_bounds__(kWarps * 32, row_fwd_min_blocks<P, PRE>()) k_r
           v[e] = c.live ? row_weight<PRE>(a, term, c.iw, c.y, pos_first<P>(c.t, e), raw[e]) : make_float2(0.f, 0.f);
       }
     }
+    if (term + 1 == nterm) chain_next();
     fft_fwd<P>(v, c.t, c.tw, c.line);
     if (c.live) {
       float2* dst = a.t1 + (long long)term * a.tstride + (c.bl * a.d.NY + c.y) * P::N;
@@ -519,7 +520,7 @@ __global__ void __launch_bounds__(kWarps * 32, multi_term(POST) && (P::E == 16 |
     k_row_inv(const SpecArgs a, int nchunk, int post_taper) {
   extern __shared__ float2 smem[];
   RowCtx<P> c(a, smem, nchunk);
-  chain_next();
+  if (a.early) chain_next();
   load_stage_tw<P>(c.tw, a.twx);
   chain_wait();
   prefetch_next_ctas<P::N, RowGeo<P>::ROWS>(a, a.t2, true, nchunk);  // the first term of a later CTA
@@ -663,6 +664,7 @@ __global__ void __launch_bounds__(kWarps * 32, multi_term(POST) && (P::E == 16 |
     }
     term = nxt;
   }
+  chain_next();
   if (!c.live) return;
   float2* dst = a.out + (c.b * a.d.NY + c.y) * P::N;
   float2* dst2 = kPair ? a.out2 + (c.b * a.d.NY + c.y) * P::N : nullptr;
@@ -813,7 +815,7 @@ template <class P, int QM>
 __global__ void __launch_bounds__(kWarps * 32, ColGeo<P>::kMinBlocksA) k_col_a(const SpecArgs a, int nxt) {
   extern __shared__ float2 smem[];
   ColCtx<P> c(a, smem, nxt);
-  chain_next();
+  if (a.early) chain_next();
   load_stage_tw<P>(c.tw, a.twy);
   chain_wait();
   cols_to_tile<P>(c.tile, a.t1, a, c.b, c.x0);
@@ -858,6 +860,7 @@ __global__ void __launch_bounds__(kWarps * 32, ColGeo<P>::kMinBlocksA) k_col_a(c
       for (int e = 0; e < P::E; ++e) v[e] = cmul(psi[e], v[e]);
     }
     __syncthreads();  // the previous term's tile has been stored
+    if (term + 1 == a.nterm) chain_next();
     fft_inv<P>(v, c.t, c.tw, c.line);
     __syncwarp();
 #pragma unroll
@@ -891,7 +894,7 @@ __global__ void __launch_bounds__(kWarps * 32, ColGeo<P>::kMinBlocks) k_col_b(co
   ColCtx<P> c(a, smem, nxt);
   float2* tiles[2] = {c.tile, c.tw + tw_size<P>()};
   const long long lineoff = (long long)c.col * ColGeo<P>::LINE;
-  chain_next();
+  if (a.early) chain_next();
   load_stage_tw<P>(c.tw, a.twy);
   chain_wait();
   const int xq = c.x < a.d.NX ? c.x : 0;
@@ -926,6 +929,7 @@ __global__ void __launch_bounds__(kWarps * 32, ColGeo<P>::kMinBlocks) k_col_b(co
     }
   }
   __syncthreads();
+  chain_next();
   fft_inv<P>(acc, c.t, c.tw, c.line);
   __syncwarp();
 #pragma unroll
@@ -1041,7 +1045,7 @@ __global__ void __launch_bounds__(kWarps * 32, col_tma_min_blocks<P>(kQT, false)
     tma::mbar_init(&bar[2], 1);
     tma::fence_mbar_init();
   }
-  chain_next();
+  if (a.early) chain_next();
   load_stage_tw<P>(tw, a.twy);
   chain_wait();
   __syncthreads();
@@ -1122,6 +1126,7 @@ __global__ void __launch_bounds__(kWarps * 32, col_tma_min_blocks<P>(kQT, false)
     }
   }
   // no load is pending: buffer 0 holds the inverse transform's exchanges, buffer 1 the result
+  chain_next();
   fft_inv<P>(acc, t, tw, tiles[0] + col * P::N);
 #pragma unroll
   for (int e = 0; e < P::E; ++e) tiles[1][tma::swz_tile<C::LX>(pos_first<P>(t, e), col)] = acc[e];
@@ -1186,7 +1191,7 @@ __global__ void __launch_bounds__(kWarps * 32, col_tma_min_blocks<P>(kQT, true))
     for (int k = 0; k < 1 + C::SLOTS; ++k) tma::mbar_init(&bar[k], 1);
     tma::fence_mbar_init();
   }
-  chain_next();
+  if (a.early) chain_next();
   load_stage_tw<P>(tw, a.twy);
   chain_wait();
   __syncthreads();
@@ -1278,6 +1283,7 @@ __global__ void __launch_bounds__(kWarps * 32, col_tma_min_blocks<P>(kQT, true))
 #pragma unroll
       for (int e = 0; e < P::E; ++e) v[e] = cmul(psi[e], v[e]);
     }
+    if (term + 1 == nterm) chain_next();
     fft_inv<P>(v, t, tw, line);
     stage_free();
     if constexpr (kQT) {  // every lane has read this term's factors
@@ -1365,6 +1371,17 @@ int resident_ctas(K kernel, size_t smem) {
   return done[key] = per * sms;
 }
 
+// Launches a column pass; its early start as for the row passes below.
+template <class K, class... Args>
+cudaError_t launch_cols(K kernel, unsigned grid, size_t sm, cudaStream_t s, const SpecArgs& a, Args... args) {
+  cudaError_t e = opt_in_smem(kernel, sm);
+  if (e != cudaSuccess) return e;
+  SpecArgs b = a;
+  const int res = resident_ctas(kernel, sm);
+  b.early = res > 0 && grid > (unsigned)res;
+  return launch_chained(a.d.chained, kernel, grid, kWarps * 32, sm, s, b, args...);
+}
+
 // Launches a row pass with its L2 hint distance: one wave of resident CTAs
 // ahead, when the grid has more than one wave (NSPS step at 256 x 256 x 128:
 // 0.191 -> 0.187 ms).  The same hint for the TMA column passes' first tile
@@ -1374,11 +1391,9 @@ cudaError_t launch_hinted(K kernel, unsigned grid, size_t sm, cudaStream_t s, co
   cudaError_t e = opt_in_smem(kernel, sm);
   if (e != cudaSuccess) return e;
   SpecArgs b = a;
-  b.pf_ctas = 0;
-  if (FWIX_NEXT_WAVE_HINTS) {
-    const int res = resident_ctas(kernel, sm);
-    if (res > 0 && grid > (unsigned)res) b.pf_ctas = res;
-  }
+  const int res = resident_ctas(kernel, sm);
+  b.early = res > 0 && grid > (unsigned)res;
+  b.pf_ctas = FWIX_NEXT_WAVE_HINTS && b.early ? res : 0;
   return launch_chained(a.d.chained, kernel, grid, kWarps * 32, sm, s, b, args...);
 }
 
@@ -1477,8 +1492,7 @@ cudaError_t col_type_a_tma(const SpecArgs& a, int qmode, cudaStream_t s) {
   if (e == cudaSuccess && qtile) e = qtab_map(&tq, a.ptab, a.ptab_ny, a.ptab_nx, (long long)a.nterm * a.d.nw, C::LX, ColTma<P>::QROWS);
   if (e != cudaSuccess) return e;
 #define FWIX_FAST_CAT(Q, QT)                                                                          \
-  e = opt_in_smem(k_col_a_tma<P, Q, QT>, sm);                                                         \
-  if (e == cudaSuccess) e = launch_chained(a.d.chained, k_col_a_tma<P, Q, QT>, grid, kWarps * 32, sm, s, a, nxt, tin, tout, tq);
+  e = launch_cols(k_col_a_tma<P, Q, QT>, grid, sm, s, a, nxt, tin, tout, tq);
   switch (qmode) {
     case Q_PS_FWD:
       if (qtile) {
@@ -1514,8 +1528,7 @@ cudaError_t col_type_a(const SpecArgs& a, int qmode, cudaStream_t s) {
   cudaError_t e;
 #define FWIX_FAST_CA(Q)                                                           \
   case Q:                                                                         \
-    e = opt_in_smem(k_col_a<P, Q>, sm);                                           \
-    if (e == cudaSuccess) e = launch_chained(a.d.chained, k_col_a<P, Q>, grid, kWarps * 32, sm, s, a, nxt); \
+    e = launch_cols(k_col_a<P, Q>, grid, sm, s, a, nxt); \
     break;
   switch (qmode) {
     FWIX_FAST_CA(Q_PS_FWD)
@@ -1545,8 +1558,7 @@ cudaError_t col_type_b_tma(const SpecArgs& a, int qmode, cudaStream_t s) {
   if (e == cudaSuccess && qtile) e = qtab_map(&tq, a.ptab, a.ptab_ny, a.ptab_nx, (long long)a.nterm * a.d.nw, C::LX, ColTma<P>::QROWS);
   if (e != cudaSuccess) return e;
 #define FWIX_FAST_CBT(Q, QT)                                                                          \
-  e = opt_in_smem(k_col_b_tma<P, Q, QT>, sm);                                                         \
-  if (e == cudaSuccess) e = launch_chained(a.d.chained, k_col_b_tma<P, Q, QT>, grid, kWarps * 32, sm, s, a, nxt, tin, tout, tq);
+  e = launch_cols(k_col_b_tma<P, Q, QT>, grid, sm, s, a, nxt, tin, tout, tq);
   switch (qmode) {
     case Q_PS_FWD:
       if (qtile) {
@@ -1582,8 +1594,7 @@ cudaError_t col_type_b(const SpecArgs& a, int qmode, cudaStream_t s) {
   cudaError_t e;
 #define FWIX_FAST_CB(Q)                                                           \
   case Q:                                                                         \
-    e = opt_in_smem(k_col_b<P, Q>, sm);                                           \
-    if (e == cudaSuccess) e = launch_chained(a.d.chained, k_col_b<P, Q>, grid, kWarps * 32, sm, s, a, nxt); \
+    e = launch_cols(k_col_b<P, Q>, grid, sm, s, a, nxt); \
     break;
   switch (qmode) {
     FWIX_FAST_CB(Q_PS_FWD)

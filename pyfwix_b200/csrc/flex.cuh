@@ -26,6 +26,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <tuple>
 #include <type_traits>
 #include <utility>
 
@@ -314,7 +315,7 @@ __global__ void __launch_bounds__(S::ROW_THREADS, min_blocks<S>(S::ROW_THREADS, 
   float2* const buf1 = buf0 + d.rows() * row_ls(d.n(), S::RT);
   const RowCtx<S> c(a, d);
   const RowPlace<S, false> w(d);
-  chain_next();
+  if (a.early) chain_next();
   fill_twiddles(tw, a.twx, RT, d.rb(), d.ra(), d.row_threads());
   chain_wait();
   constexpr bool kSmooth = CLS == C_SMOOTH;
@@ -419,6 +420,7 @@ __global__ void __launch_bounds__(S::ROW_THREADS, min_blocks<S>(S::ROW_THREADS, 
       __syncthreads();
       src = buf1;
     }
+    if (term + 1 == nterm) chain_next();
     const float2* twl = tw + (d.rb() - 1) * RT;
     stage_a(d, [&](auto rc) {
       constexpr int R = decltype(rc)::value;
@@ -451,7 +453,7 @@ __global__ void __launch_bounds__(S::ROW_THREADS, min_blocks<S>(S::ROW_THREADS, 
   float2* const buf1 = buf0 + d.rows() * row_ls(d.n(), d.ra());
   const RowCtx<S> c(a, d);
   const RowPlace<S, true> w(d);
-  chain_next();
+  if (a.early) chain_next();
   fill_twiddles(tw, a.twx, d.ra(), d.rb(), RT, d.row_threads());
   chain_wait();
   // kDeriv: the sum of w_r' C_r T_r beside the step's own
@@ -552,6 +554,7 @@ __global__ void __launch_bounds__(S::ROW_THREADS, min_blocks<S>(S::ROW_THREADS, 
       for (int r = 0; r < RT; ++r) acc[r] = v[r];
     }
   }
+  chain_next();
   if (!c.live) return;
   const long long roff = (c.b * a.d.NY + c.y) * d.n();
   const float ty = post_taper ? a.tapy[c.y] : 1.f;
@@ -624,18 +627,28 @@ __device__ __forceinline__ void col_first(const SpecArgs& a, const Dim<S>& d, co
     for (int i = threadIdx.x; i < d.cols() * d.na(); i += d.col_threads()) {
       const int cc = i & (d.cols() - 1), j = i >> d.sh();
       if (c.x0 + cc >= a.d.NX) continue;
+      const int o = j * a.d.NX + cc, step = d.na() * a.d.NX;
       float2 u[R];
 #pragma unroll
-      for (int r = 0; r < R; ++r) u[r] = src[(j + r * d.na()) * a.d.NX + cc];
+      for (int r = 0; r < R; ++r) u[r] = src[o + r * step];
       if (cp) {
 #pragma unroll
-        for (int r = 0; r < R; ++r) cp[(j + r * d.na()) * a.d.NX + cc] = cscale(u[r], scale);
+        for (int r = 0; r < R; ++r) cp[o + r * step] = cscale(u[r], scale);
       }
       Dft<R, false>::run(u);
 #pragma unroll
       for (int r = 0; r < R; ++r) dst[((j * R + r) << d.sh()) + cc] = u[r];
     }
   });
+}
+// Hints into L2 the CTA's columns of slice-local b of a later term: one hint per row
+// segment.
+template <class S>
+__device__ __forceinline__ void col_prefetch(const SpecArgs& a, const Dim<S>& d, const ColCtx<S>& c,
+                                             const float2* in) {
+  const float2* p = in + c.b * a.d.slice + c.x0;
+  for (int y = threadIdx.x; y < d.n(); y += d.col_threads())
+    asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p + y * a.d.NX));
 }
 // Middle stage, src -> dst; span = the first stage's radix.
 template <bool INV, class S>
@@ -672,11 +685,17 @@ __device__ __forceinline__ void col_last(const SpecArgs& a, const Dim<S>& d, con
 #pragma unroll
       for (int r = 1; r < R; ++r) u[r] = cmul_conj(u[r], twl[(r - 1) * d.na() + j]);
       Dft<R, true>::run(u);
+      float2* const o = dst + j * a.d.NX + cc;
+      const int step = d.na() * a.d.NX;
+      if (add) {
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        float2* q = dst + (j + r * d.na()) * a.d.NX + cc;
-        float2 v = scale != 1.f ? cscale(u[r], scale) : u[r];
-        *q = add ? cadd(*q, v) : v;
+        for (int r = 0; r < R; ++r) o[r * step] = cadd(o[r * step], cscale(u[r], scale));
+      } else if (scale != 1.f) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) o[r * step] = cscale(u[r], scale);
+      } else {
+#pragma unroll
+        for (int r = 0; r < R; ++r) o[r * step] = u[r];
       }
     }
   });
@@ -704,10 +723,19 @@ __device__ __forceinline__ void col_factors(const SpecArgs& a, const Dim<S>& d, 
       const float2 sr = a.sref[t * a.d.nw + c.iw];
       flip = !(a.w2[c.iw] * (sr.y - a.eps * sr.x) > 0.f);
     }
+    // a thread's j < nt, so most of its rows know their side of n / 2: they step from
+    // two bases by a multiple of the row pitch instead of a minimum and a product each
+    const int step = d.nt() * a.ptab_sy;
+    const float2* const up = p + c.j * a.ptab_sy;
+    const float2* const down = p + (d.n() - c.j) * a.ptab_sy;
 #pragma unroll
     for (int r = 0; r < RT; ++r) {
-      const int ky = c.j + r * d.nt();
-      q[r] = p[min(ky, d.n() - ky) * a.ptab_sy];
+      if (2 * r + 2 <= RT)  // j + r nt < (r + 1) nt <= n / 2
+        q[r] = up[r * step];
+      else if (2 * r >= RT)
+        q[r] = down[-(r * step)];
+      else
+        q[r] = p[min(c.j + r * d.nt(), d.n() - c.j - r * d.nt()) * a.ptab_sy];
     }
     if (flip) {
 #pragma unroll
@@ -740,7 +768,7 @@ __global__ void __launch_bounds__(S::COL_THREADS, min_blocks<S>(S::COL_THREADS, 
   float2* const buf0 = sm + d.fwd_rows_tw() + d.inv_rows_tw();
   float2* const buf1 = buf0 + (d.n() << d.sh());
   const ColCtx<S> c(a, d);
-  chain_next();
+  if (a.early) chain_next();
   col_twiddles(a, d, tw);
   chain_wait();
   // the zeroth Born order's filter is the identity: its output is the input,
@@ -775,6 +803,7 @@ __global__ void __launch_bounds__(S::COL_THREADS, min_blocks<S>(S::COL_THREADS, 
       __syncthreads();
       dst = buf1;
     }
+    if (term + 1 == a.nterm) chain_next();
     col_last(a, d, c, itw + (d.rb() - 1) * RT, dst, a.t2 + (long long)term * a.tstride, 0, 1.f);
   }
 }
@@ -790,7 +819,7 @@ __global__ void __launch_bounds__(S::COL_THREADS, min_blocks<S>(S::COL_THREADS, 
   float2* const buf0 = sm + d.fwd_rows_tw() + d.inv_rows_tw();
   float2* const buf1 = buf0 + (d.n() << d.sh());
   const ColCtx<S> c(a, d);
-  chain_next();
+  if (a.early) chain_next();
   col_twiddles(a, d, tw);
   chain_wait();
   float2 acc[RT];
@@ -799,6 +828,7 @@ __global__ void __launch_bounds__(S::COL_THREADS, min_blocks<S>(S::COL_THREADS, 
   for (int term = 0; term < a.nterm; ++term) {
     float2* src = (d.rb() == 1 && (term & 1)) ? buf1 : buf0;
     col_first(a, d, c, a.t1 + (long long)term * a.tstride, src);
+    if (term + 1 < a.nterm) col_prefetch(a, d, c, a.t1 + (long long)(term + 1) * a.tstride);
     __syncthreads();
     if (d.rb() > 1) {
       col_mid<false>(d, tw, buf0, buf1, d.ra());
@@ -813,6 +843,7 @@ __global__ void __launch_bounds__(S::COL_THREADS, min_blocks<S>(S::COL_THREADS, 
       for (int r = 0; r < RT; ++r) acc[r] = cadd(acc[r], cmul(v[r], q[r]));
     }
   }
+  chain_next();
   // the last term left its samples in buf1 (three stages) or in buf[(nterm - 1) & 1]
   float2* dst = (d.rb() == 1 && (a.nterm & 1)) ? buf1 : buf0;
   if (c.ok) {
@@ -841,7 +872,7 @@ __global__ void __launch_bounds__(S::COL_THREADS, min_blocks<S>(S::COL_THREADS, 
   float2* const buf0 = sm + d.fwd_rows_tw() + d.inv_rows_tw();
   float2* const buf1 = buf0 + (d.n() << d.sh());
   const ColCtx<S> c(a, d);
-  chain_next();
+  if (a.early) chain_next();
   col_twiddles(a, d, tw);
   chain_wait();
   const long long off = c.b * a.d.slice + c.x;
@@ -921,30 +952,47 @@ inline Geo col_geo(const SpecArgs& a, const Line& p, unsigned* threads, size_t* 
   return g;
 }
 
-// Opts a kernel in to the shared memory of its launch, once per (kernel, device, size).
+// Opts a kernel in to the shared memory of its launch, once per (kernel, device, size),
+// and gives the CTAs of it that the device holds at once.
 template <class K>
-cudaError_t opt_in(K kernel, size_t bytes) {
+cudaError_t opt_in(K kernel, unsigned threads, size_t bytes, int* resident) {
   static std::mutex mu;
-  static std::map<std::pair<const void*, int>, size_t> done;
+  static std::map<std::tuple<const void*, int, size_t>, int> done;
+  static std::map<std::pair<const void*, int>, size_t> most;
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  const auto key = std::make_pair((const void*)kernel, dev);
+  const auto key = std::make_tuple((const void*)kernel, dev, bytes * 2048 + threads);
   std::lock_guard<std::mutex> lock(mu);
   auto it = done.find(key);
-  if (it != done.end() && it->second >= bytes) return cudaSuccess;
+  if (it != done.end()) {
+    *resident = it->second;
+    return cudaSuccess;
+  }
+  size_t& m = most[std::make_pair((const void*)kernel, dev)];
   e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-  if (e == cudaSuccess && bytes > 48 * 1024)
+  if (e == cudaSuccess && bytes > 48 * 1024 && bytes > m)
     e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (e == cudaSuccess) done[key] = bytes;
-  return e;
+  if (e != cudaSuccess) return e;
+  m = std::max(m, bytes);
+  int per = 0, sms = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, (int)threads, bytes) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+    cudaGetLastError();
+    per = 0;
+  }
+  *resident = done[key] = per * sms;
+  return cudaSuccess;
 }
 
 template <class K, class... Args>
 cudaError_t launch(K kernel, unsigned grid, unsigned threads, size_t smem, cudaStream_t s, const SpecArgs& a,
                    Args... args) {
-  cudaError_t e = opt_in(kernel, smem);
-  if (e == cudaSuccess) e = launch_chained(a.d.chained, kernel, grid, threads, smem, s, a, args...);
+  int res = 0;
+  cudaError_t e = opt_in(kernel, threads, smem, &res);
+  SpecArgs b = a;
+  b.early = res > 0 && grid > (unsigned)res;
+  if (e == cudaSuccess) e = launch_chained(a.d.chained, kernel, grid, threads, smem, s, b, args...);
   if (e == cudaSuccess) count_launch();
   return e != cudaSuccess ? e : cudaGetLastError();
 }

@@ -139,26 +139,37 @@ struct SpecArgs {
   const float2* rf_tab;
   const float2* rf_f1;
   const float2* rf_f2;
+  // chained passes: let the next kernel's CTAs in from the start (a grid of more than
+  // one wave) instead of at the last stage
+  int early;
   // register-resident row passes: each CTA hints into L2 the first input rows
   // of the CTA pf_ctas launch positions later, the one that takes its place
   // once every resident CTA has run (0: none)
   int pf_ctas;
 };
 
-// Chained launches.  A kernel launched with chained set may start, CTA by CTA, while
-// the kernel before it on the stream drains: up to chain_wait() it may only touch
-// what no kernel on the stream writes (a plan's twiddle tables, its own shared
-// memory); chain_wait() returns once the kernel before it has completed with its
-// writes visible (at once for an ordinary launch).  Every thread calls both,
-// chain_next() first.  The prologue and the launch gap (1 - 2 us of kernels of 5 -
-// 30 us at 128 x 128 and below) then go under the kernel before: modelling at 128 x
-// 128 x 64 2432 -> 2042 us, an NSPS step and its adjoint at 105 x 90 x 24 59 -> 46
-// us, the Born pair at 256 x 256 x 128 13.71 -> 13.35 ms.  Instances that share the
+// Chained launches.  A kernel launched with chained set may start, CTA by CTA, once
+// every CTA of the kernel before it on the stream has called chain_next() or ended:
+// up to chain_wait() it may only touch what no kernel on the stream writes (a plan's
+// twiddle tables, its own shared memory); chain_wait() returns once the kernel before
+// it has completed with its writes visible (at once for an ordinary launch).  Every
+// thread calls chain_wait().  The prologue and the launch gap (1 - 2 us of kernels of
+// 5 - 30 us at 128 x 128 and below) then go under the kernel before: modelling at 128
+// x 128 x 64 2432 -> 2042 us, the Born pair at 256 x 256 x 128 13.71 -> 13.35 ms.  A grid
+// of more than a wave calls chain_next() at its start (SpecArgs::early; at the last
+// stage instead the Born pair takes 12.75 ms for 12.46), a smaller one at its last
+// stage: CTAs placed early fill the SMs that run dry first, and the next grid, of less
+// than a wave too, would run on a part of the GPU (NSPS step and adjoint at 105 x 90 x
+// 24, queued back to back, 54.7 us early and 39.1 late).  Instances that share the
 // GPU over several streams are not chained (fwix_sweep): there the waiting CTAs hold
 // places that the other streams' kernels could use (6.31 -> 6.48 ms, four shots).
 #ifdef __CUDACC__
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// chain_next() for a grid of plain threads that exceeds what the SMs hold at once.
+__device__ __forceinline__ void chain_next_if_large() {
+  if (gridDim.x * gridDim.y > 148u * (2048u / (blockDim.x * blockDim.y))) chain_next();
+}
 
 template <class... KArgs, class... Args>
 cudaError_t launch_chained(bool chained, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,

@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(kCells * kGroups)
     k_reflect(Dims d, int adjoint, const float2* __restrict__ s0, const float2* __restrict__ s1,
               const float2* __restrict__ r0, const float2* __restrict__ r1, long long mw,
               const float2* __restrict__ in, float2* __restrict__ out) {
-  chain_next();
+  chain_next_if_large();
   chain_wait();
   const Cell c = this_cell(d);
   // one model for every frequency: the first group forms each cell's coefficient once
@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(kCells * kGroups)
 __global__ void __launch_bounds__(kCells * kGroups)
     k_ic_fwd(Dims d, const float2* __restrict__ bg, const float2* __restrict__ image, long long img_w,
              float2* __restrict__ wfld) {
-  chain_next();
+  chain_next_if_large();
   chain_wait();
   const Cell c = this_cell(d);
   if (!c.ok) return;
@@ -128,7 +128,7 @@ template <bool S1>
 __global__ void __launch_bounds__(kCells * kGroups)
     k_ic_adj(Dims d, const float2* __restrict__ bg, const float2* __restrict__ wfld, float2* __restrict__ image,
              int add, int wsum) {
-  chain_next();
+  chain_next_if_large();
   chain_wait();
   const Cell c = this_cell(d);
   float2 acc[1] = {make_float2(0.f, 0.f)};
@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(kCells * kGroups)
                   float2* dm1, float2* dm2, float2* dm3, long long dm_w, float2* dr, int add,
                   const float2* __restrict__ bg, float2* __restrict__ wf, const float2* __restrict__ bg2,
                   const float2* __restrict__ wf2) {
-  chain_next();
+  chain_next_if_large();
   chain_wait();
   const Cell c = this_cell(d);
   const int ns = S1 ? 1 : d.ns;
@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(256)
                  const float2* __restrict__ r0, const float2* __restrict__ r1, const float2* __restrict__ dm0,
                  const float2* __restrict__ dm1, const float2* __restrict__ dm2, const float2* __restrict__ dm3,
                  float2* __restrict__ tab) {
-  chain_next();
+  chain_next_if_large();
   chain_wait();
   const long long n = (long long)d.ny * d.nx;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
@@ -329,7 +329,7 @@ template <bool S1>
 __global__ void __launch_bounds__(kCells * kGroups)
     k_image_acc(Dims d, const float2* __restrict__ S, const float2* __restrict__ R, float* __restrict__ img,
                 int add) {
-  chain_next();
+  chain_next_if_large();
   chain_wait();
   const Cell c = this_cell(d);
   float2 acc[1] = {make_float2(0.f, 0.f)};
@@ -352,7 +352,7 @@ template <bool S1>
 __global__ void __launch_bounds__(kCells * kGroups)
     k_image_acc2(Dims d, int ny2, int nx2, const float2* __restrict__ S, const float2* __restrict__ R1,
                  const float2* __restrict__ R2, float* __restrict__ img1, float* __restrict__ img2, int add) {
-  chain_next();
+  chain_next_if_large();
   chain_wait();
   const Cell c = this_cell(d);
   float2 acc[1] = {make_float2(0.f, 0.f)};
@@ -394,7 +394,7 @@ __global__ void k_axpy(long long n, const float2* __restrict__ x, float2* __rest
 // wfld[shot, w, y, x] += sum_k weight_k * traces[trace_k, w] for each listed cell.
 __global__ void __launch_bounds__(256) k_inject(Dims d, InjectLevel L, const float2* __restrict__ traces,
                                                 float2* wfld) {
-  chain_next();
+  chain_next_if_large();
   chain_wait();
   __shared__ float2 tile[32][33];
   const int e0 = blockIdx.x * 32, w0 = blockIdx.y * 32;
@@ -421,7 +421,7 @@ __global__ void __launch_bounds__(256) k_inject(Dims d, InjectLevel L, const flo
 // traces[t, w] += sum of the four corner weights times the wavefield.
 __global__ void __launch_bounds__(256) k_record(Dims d, InjectLevel L, const float2* __restrict__ wfld,
                                                 float2* traces) {
-  chain_next();
+  chain_next_if_large();
   chain_wait();
   __shared__ float2 tile[32][33];
   const int e0 = blockIdx.x * 32, w0 = blockIdx.y * 32;

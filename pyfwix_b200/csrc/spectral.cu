@@ -419,7 +419,7 @@ __global__ void k_phase_shift(const SpecArgs a, const float2* __restrict__ in, f
 
 template <int W>
 __global__ void k_weight(const SpecArgs a, int t, const float2* __restrict__ in, float2* out, int add) {
-  chain_next();
+  chain_next_if_large();
   chain_wait();
   const long long n = a.d.wfld;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
@@ -464,7 +464,7 @@ cudaError_t launch_phase_shift(const SpecArgs& a, int mode, const float2* sref_w
 // and the store, and no index divisions.
 constexpr int kTableRows = 8;  // warps of a CTA
 __global__ void __launch_bounds__(256) k_phase_table(const SpecArgs a, int nblk, float2* dst) {
-  chain_next();
+  chain_next_if_large();
   chain_wait();
   const bool ky_fast = a.ptab_sy == 1;
   const int nf = ky_fast ? a.ptab_ny : a.ptab_nx, ns = ky_fast ? a.ptab_nx : a.ptab_ny;
@@ -497,7 +497,7 @@ cudaError_t launch_select(const SpecArgs& a, int value, const float2* in, float2
 }
 
 __global__ void k_scat_table(const SpecArgs a, float2* dst) {
-  chain_next();
+  chain_next_if_large();
   chain_wait();
   const long long n = (long long)a.nterm * a.d.slice;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
