@@ -23,6 +23,7 @@ workload; the reference itself has no CPU implementation of this path.
 from __future__ import annotations
 
 import argparse
+import gc
 import json
 import math
 import os
@@ -808,7 +809,10 @@ def main():
         fwi["shots_across_ranks"] = sh
         from pyfwix_b200.fwi import clear_plan_cache
         clear_plan_cache()  # the FWI plan's phase cache is not needed by the timings below
-        torch.cuda.empty_cache()
+    # nor is what earlier timings left in reference cycles (plans, fields): the batch
+    # below needs the room
+    gc.collect()
+    torch.cuda.empty_cache()
     config1 = config1_timing(device, autotune=not a.no_autotune) if not a.no_config1 else None
     if ws == 1 and not a.no_batched:
         batched = batched_timing(device, nshots=a.batched_shots, nz=a.batched_nz, nstreams=a.batched_streams)

@@ -17,10 +17,13 @@
 // its stride, is a contiguous 8 LX bytes (no bank conflicts without a swizzle)
 // and HBM is touched in segments of the same length.
 //
-// What bounds them: shared-memory and issue throughput, as for the compile-time
-// plans; the per-warp passes that they replace (spectral.cu) crossed shared
-// memory 7 to 9 times per sample and term, in stages of radix 8 at most with a
-// part of the lanes idle.
+// What bounds them: the latency of a term's global loads at 14 - 24 warps per SM, then
+// the L1 data pipe (8-byte accesses), 20 - 37 % of DRAM bandwidth.  us per pass, with
+// the per-warp passes of spectral.cu that these replace (7 to 9 shared-memory crossings
+// per sample and term, radix 8 at most, a part of the lanes idle): PSPI continuation and
+// its adjoint over six levels at 200 x 168 x 40 1569 -> 720; four uneven shots (270, 216,
+// 160, 135) imaged 11580 -> 5830; the Born pair at 135 x 120 x 40 on two shots 6240 ->
+// 3060.
 #pragma once
 #include <algorithm>
 #include <cstring>

@@ -461,7 +461,8 @@ cudaError_t launch_phase_shift(const SpecArgs& a, int mode, const float2* sref_w
 // same arithmetic as the in-kernel evaluation (k depends on |index| only).  A CTA
 // takes kTableRows rows (of the slower of the two indices) of one (ref, w) slice, a
 // warp a row, so that a factor costs its root, exponential or sine, its table reads
-// and the store, and no index divisions.
+// and the store, and no index divisions (64-bit ones per factor: 80 us at 384 x 384 x 96
+// with four references; now 47, of which the stores take 17).
 constexpr int kTableRows = 8;  // warps of a CTA
 __global__ void __launch_bounds__(256) k_phase_table(const SpecArgs a, int nblk, float2* dst) {
   chain_next_if_large();
