@@ -749,7 +749,7 @@ struct ColCtx {
 
 // Coalesced copy of the CTA's columns of slice-local b between HBM and the tile.
 template <class P>
-__device__ __forceinline__ void cols_to_tile(float2* tile, const float2* __restrict__ g, const SpecArgs& a,
+__device__ __forceinline__ void cols_to_tile(float2* tile, const float2* g, const SpecArgs& a,
                                              long long b, int x0) {
   constexpr int LX = ColGeo<P>::LX, NT = kWarps * 32;
   static_assert((LX * P::N) % NT == 0, "tile is a whole number of CTA sweeps");
@@ -872,7 +872,7 @@ __global__ void __launch_bounds__(kWarps * 32, ColGeo<P>::kMinBlocksA) k_col_a(c
 
 // Asynchronous copy of the CTA's columns of slice-local b into a tile.
 template <class P>
-__device__ __forceinline__ void cols_to_tile_async(float2* tile, const float2* __restrict__ g, const SpecArgs& a,
+__device__ __forceinline__ void cols_to_tile_async(float2* tile, const float2* g, const SpecArgs& a,
                                                    long long b, int x0) {
   constexpr int LX = ColGeo<P>::LX, NT = kWarps * 32;
   const int cc = threadIdx.x % LX, x = x0 + cc;

@@ -153,7 +153,11 @@ struct SpecArgs {
 // up to chain_wait() it may only touch what no kernel on the stream writes (a plan's
 // twiddle tables, its own shared memory); chain_wait() returns once the kernel before
 // it has completed with its writes visible (at once for an ordinary launch).  Every
-// thread calls chain_wait().  The prologue and the launch gap (1 - 2 us of kernels of
+// thread calls chain_wait().  A chained kernel takes what it reads through plain
+// pointers, never const __restrict__: that promises memory which no one writes while
+// the kernel runs, so its loads may go to the non-coherent read-only path or ahead of
+// chain_wait(), and here the kernel before still writes while this one starts.  (An
+// output that the kernel itself writes may be __restrict__.)  The prologue and the launch gap (1 - 2 us of kernels of
 // 5 - 30 us at 128 x 128 and below) then go under the kernel before: modelling at 128
 // x 128 x 64 2432 -> 2042 us, the Born pair at 256 x 256 x 128 13.71 -> 13.35 ms.  A grid
 // of more than a wave calls chain_next() at its start (SpecArgs::early; at the last

@@ -73,9 +73,9 @@ unsigned cell_blocks(const Dims& d) { return (unsigned)((d.ny * d.nx + kCells - 
 
 template <bool S1>
 __global__ void __launch_bounds__(kCells * kGroups)
-    k_reflect(Dims d, int adjoint, const float2* __restrict__ s0, const float2* __restrict__ s1,
-              const float2* __restrict__ r0, const float2* __restrict__ r1, long long mw,
-              const float2* __restrict__ in, float2* __restrict__ out) {
+    k_reflect(Dims d, int adjoint, const float2* s0, const float2* s1,
+              const float2* r0, const float2* r1, long long mw,
+              const float2* in, float2* __restrict__ out) {
   chain_next_if_large();
   chain_wait();
   const Cell c = this_cell(d);
@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(kCells * kGroups)
 }
 
 __global__ void __launch_bounds__(kCells * kGroups)
-    k_ic_fwd(Dims d, const float2* __restrict__ bg, const float2* __restrict__ image, long long img_w,
+    k_ic_fwd(Dims d, const float2* bg, const float2* image, long long img_w,
              float2* __restrict__ wfld) {
   chain_next_if_large();
   chain_wait();
@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(kCells * kGroups)
 // into image[y, x].
 template <bool S1>
 __global__ void __launch_bounds__(kCells * kGroups)
-    k_ic_adj(Dims d, const float2* __restrict__ bg, const float2* __restrict__ wfld, float2* __restrict__ image,
+    k_ic_adj(Dims d, const float2* bg, const float2* wfld, float2* __restrict__ image,
              int add, int wsum) {
   chain_next_if_large();
   chain_wait();
@@ -184,11 +184,11 @@ __device__ __forceinline__ LinCoef lin_coef(float2 s0, float2 s1, float2 r0, flo
 // one read of the four fields serves both frequency sums of a level.
 template <bool IC, bool S1, bool IC2>
 __global__ void __launch_bounds__(kCells * kGroups)
-    k_lin_reflect(Dims d, int adjoint, const float2* __restrict__ s0, const float2* __restrict__ s1,
-                  const float2* __restrict__ r0, const float2* __restrict__ r1, long long mw, float2* dm0,
+    k_lin_reflect(Dims d, int adjoint, const float2* s0, const float2* s1,
+                  const float2* r0, const float2* r1, long long mw, float2* dm0,
                   float2* dm1, float2* dm2, float2* dm3, long long dm_w, float2* dr, int add,
-                  const float2* __restrict__ bg, float2* __restrict__ wf, const float2* __restrict__ bg2,
-                  const float2* __restrict__ wf2) {
+                  const float2* bg, float2* __restrict__ wf, const float2* bg2,
+                  const float2* wf2) {
   chain_next_if_large();
   chain_wait();
   const Cell c = this_cell(d);
@@ -305,9 +305,9 @@ __global__ void __launch_bounds__(kCells * kGroups)
 // tab[ny nx + yx] = as dm0 - bs dm1 + ar dm3 - br dm2, the linearised reflection
 // that k_lin_reflect's forward forms.
 __global__ void __launch_bounds__(256)
-    k_refl_table(Dims d, int adjoint, const float2* __restrict__ s0, const float2* __restrict__ s1,
-                 const float2* __restrict__ r0, const float2* __restrict__ r1, const float2* __restrict__ dm0,
-                 const float2* __restrict__ dm1, const float2* __restrict__ dm2, const float2* __restrict__ dm3,
+    k_refl_table(Dims d, int adjoint, const float2* s0, const float2* s1,
+                 const float2* r0, const float2* r1, const float2* dm0,
+                 const float2* dm1, const float2* dm2, const float2* dm3,
                  float2* __restrict__ tab) {
   chain_next_if_large();
   chain_wait();
@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(256)
 
 template <bool S1>
 __global__ void __launch_bounds__(kCells * kGroups)
-    k_image_acc(Dims d, const float2* __restrict__ S, const float2* __restrict__ R, float* __restrict__ img,
+    k_image_acc(Dims d, const float2* S, const float2* R, float* __restrict__ img,
                 int add) {
   chain_next_if_large();
   chain_wait();
@@ -350,8 +350,8 @@ __global__ void __launch_bounds__(kCells * kGroups)
 // img2[y][x] (+)= Re sum conj(S) R2 over the model window ny2 x nx2.
 template <bool S1>
 __global__ void __launch_bounds__(kCells * kGroups)
-    k_image_acc2(Dims d, int ny2, int nx2, const float2* __restrict__ S, const float2* __restrict__ R1,
-                 const float2* __restrict__ R2, float* __restrict__ img1, float* __restrict__ img2, int add) {
+    k_image_acc2(Dims d, int ny2, int nx2, const float2* S, const float2* R1,
+                 const float2* R2, float* __restrict__ img1, float* __restrict__ img2, int add) {
   chain_next_if_large();
   chain_wait();
   const Cell c = this_cell(d);
@@ -392,7 +392,7 @@ __global__ void k_axpy(long long n, const float2* __restrict__ x, float2* __rest
 // the same element.
 
 // wfld[shot, w, y, x] += sum_k weight_k * traces[trace_k, w] for each listed cell.
-__global__ void __launch_bounds__(256) k_inject(Dims d, InjectLevel L, const float2* __restrict__ traces,
+__global__ void __launch_bounds__(256) k_inject(Dims d, InjectLevel L, const float2* traces,
                                                 float2* wfld) {
   chain_next_if_large();
   chain_wait();
@@ -419,7 +419,7 @@ __global__ void __launch_bounds__(256) k_inject(Dims d, InjectLevel L, const flo
 }
 
 // traces[t, w] += sum of the four corner weights times the wavefield.
-__global__ void __launch_bounds__(256) k_record(Dims d, InjectLevel L, const float2* __restrict__ wfld,
+__global__ void __launch_bounds__(256) k_record(Dims d, InjectLevel L, const float2* wfld,
                                                 float2* traces) {
   chain_next_if_large();
   chain_wait();

@@ -418,7 +418,7 @@ __global__ void k_phase_shift(const SpecArgs a, const float2* __restrict__ in, f
 }
 
 template <int W>
-__global__ void k_weight(const SpecArgs a, int t, const float2* __restrict__ in, float2* out, int add) {
+__global__ void k_weight(const SpecArgs a, int t, const float2* in, float2* out, int add) {
   chain_next_if_large();
   chain_wait();
   const long long n = a.d.wfld;

@@ -1,0 +1,55 @@
+"""Rules of the CUDA sources whose breach shows on the GPU only by a race or a fault,
+if at all: checked on the text of every kernel."""
+import glob
+import os
+import re
+
+import pytest
+
+from tests.conftest import ROOT
+
+CSRC = os.path.join(ROOT, "pyfwix_b200", "csrc")
+
+
+def _match(s, i, open_, close):
+    """Index behind the bracket that closes the one at i."""
+    depth = 0
+    for k in range(i, len(s)):
+        depth += (s[k] == open_) - (s[k] == close)
+        if depth == 0:
+            return k + 1
+    raise ValueError("unbalanced brackets")
+
+
+def kernels():
+    """(name, parameters, body) of every kernel, comments removed."""
+    out = []
+    for path in sorted(glob.glob(os.path.join(CSRC, "*.cu")) + glob.glob(os.path.join(CSRC, "*.cuh"))):
+        s = re.sub(r"//[^\n]*", "", open(path).read())
+        for m in re.finditer(r"__global__", s):
+            k = s.index("k_", m.end())
+            name = re.match(r"\w+", s[k:]).group()
+            p0 = s.index("(", k)
+            p1 = _match(s, p0, "(", ")")
+            b0 = s.index("{", p1)
+            out.append((os.path.basename(path) + ":" + name, s[p0:p1], s[b0:_match(s, b0, "{", "}")]))
+    return out
+
+
+KERNELS = kernels()
+CHAINED = [k for k in KERNELS if "chain_wait()" in k[2]]
+
+
+def test_kernels_are_found():
+    names = {k[0] for k in CHAINED}
+    for n in ("pointwise.cu:k_record", "spectral.cu:k_weight", "fast.cuh:k_col_b_tma", "flex.cuh:k_row_inv"):
+        assert n in names
+
+
+@pytest.mark.parametrize("name,params,body", CHAINED, ids=[k[0] for k in CHAINED])
+def test_chained_kernels_read_through_plain_pointers(name, params, body):
+    """A chained kernel runs while the kernel before it still writes: const
+    __restrict__ would promise that nobody does."""
+    for p in params.split(","):
+        assert not ("const" in p and "__restrict__" in p), p
+    assert body.index("chain_wait()") < min([body.find(t) for t in ("return", "a.in[") if t in body] or [len(body)])
