@@ -1084,14 +1084,13 @@ __global__ void __launch_bounds__(kWarps * 32, col_tma_min_blocks<P>(kQT, false)
   float2 acc[P::E];
 #pragma unroll
   for (int e = 0; e < P::E; ++e) acc[e] = make_float2(0.f, 0.f);
-  bool good = true;  // no wait of this thread has run out (checked with the next barrier that can)
   for (int term = 0; term < a.nterm; ++term) {
     const int buf = term & 1;
     if (threadIdx.x == 0 && term + 1 < a.nterm) issue(term + 1, buf ^ 1);
     constexpr bool kQ = !kQT && QM != Q_KPOW;
     float2 q[kQ ? P::E : 1];
     if constexpr (kQ) col_factors<P, QM>(a, term, iw, xq, t, q);
-    good = tma::mbar_wait(&bar[buf], (unsigned)(term >> 1) & 1u) && good;
+    bool good = tma::mbar_wait(&bar[buf], (unsigned)(term >> 1) & 1u);
     if (!__syncthreads_and(good)) {
       bail(term);
       return;
@@ -1120,9 +1119,15 @@ __global__ void __launch_bounds__(kWarps * 32, col_tma_min_blocks<P>(kQT, false)
       for (int e = 0; e < P::E; ++e) acc[e] = cadd(acc[e], cmul(v[e], q[e]));
     }
     tma::fence_proxy_async();  // the exchanges and phase reads precede the next loads into their places
-    __syncthreads();
     if constexpr (kOwn) {
+      // a phase tile that has not landed keeps its barrier: nothing is loaded over it
+      if (!__syncthreads_and(good)) {
+        bail(term);
+        return;
+      }
       if (threadIdx.x == 0) issue_q(term + 1);
+    } else {
+      __syncthreads();
     }
   }
   // no load is pending: buffer 0 holds the inverse transform's exchanges, buffer 1 the result
@@ -1131,14 +1136,7 @@ __global__ void __launch_bounds__(kWarps * 32, col_tma_min_blocks<P>(kQT, false)
 #pragma unroll
   for (int e = 0; e < P::E; ++e) tiles[1][tma::swz_tile<C::LX>(pos_first<P>(t, e), col)] = acc[e];
   tma::fence_proxy_async();
-  if constexpr (kOwn) {
-    if (!__syncthreads_and(good)) {
-      if (threadIdx.x == 0) atomicAdd(a.err, 1u);
-      return;
-    }
-  } else {
-    __syncthreads();
-  }
+  __syncthreads();
   if (threadIdx.x == 0) {
 #pragma unroll
     for (int k = 0; k < C::NBOX; ++k) tma::store_3d(&tout, x0, k * C::ROWS, (int)b, tiles[1] + k * C::ROWS * C::LX);

@@ -53,3 +53,22 @@ def test_chained_kernels_read_through_plain_pointers(name, params, body):
     for p in params.split(","):
         assert not ("const" in p and "__restrict__" in p), p
     assert body.index("chain_wait()") < min([body.find(t) for t in ("return", "a.in[") if t in body] or [len(body)])
+
+
+TMA = [k for k in KERNELS if "mbar_wait(" in k[2]]
+
+
+@pytest.mark.parametrize("name,params,body", TMA, ids=[k[0] for k in TMA])
+def test_tma_kernels_leave_with_no_load_in_flight(name, params, body):
+    """A CTA that gives up on a wait lets its own loads land first (bail), and no
+    barrier is armed again before the wait on it was checked by the whole CTA."""
+    exits = [m.start() for m in re.finditer(r"__syncthreads_and\(", body)]
+    assert exits
+    for i in exits:
+        block = body[body.index("{", i):]
+        block = block[:_match(block, 0, "{", "}")]
+        assert "bail(" in block and "return" in block, block
+    armed = [m.start() for m in re.finditer(r"issue_q\(term \+", body)]
+    for i in armed:
+        wait = max(body.rfind(w, 0, i) for w in ("= tma::mbar_wait(&bar[2]", "= wait_q("))
+        assert wait >= 0 and "__syncthreads_and(" in body[wait:i], body[wait:i]
