@@ -1240,7 +1240,10 @@ __global__ void __launch_bounds__(kWarps * 32, col_tma_min_blocks<P>(kQT, true))
       tma::store_commit();
     }
   };
-  auto stage_free = [&]() {  // the previous store has read the staging tile
+  // The previous store has read the staging tile; every lane's phase reads precede
+  // the load that takes their slot next (the fence: they went by the generic proxy).
+  auto stage_free = [&]() {
+    if constexpr (kQT) tma::fence_proxy_async();
     if (threadIdx.x == 0) tma::store_wait_read();
     __syncthreads();
   };

@@ -72,3 +72,19 @@ def test_tma_kernels_leave_with_no_load_in_flight(name, params, body):
     for i in armed:
         wait = max(body.rfind(w, 0, i) for w in ("= tma::mbar_wait(&bar[2]", "= wait_q("))
         assert wait >= 0 and "__syncthreads_and(" in body[wait:i], body[wait:i]
+
+
+def test_phase_slots_are_fenced_before_their_next_load():
+    """A phase tile is read by plain loads and overwritten by TMA: the reading lanes pass
+    a proxy fence and a CTA barrier in between."""
+    body = {k[0]: k[2] for k in KERNELS}
+    a = body["fast.cuh:k_col_a_tma"]
+    free = a[a.index("auto stage_free"):]
+    free = free[:free.index("};")]
+    assert 0 <= free.find("fence_proxy_async()") < free.find("__syncthreads()")
+    read, issue = a.index("qr[T::qat("), a.index("issue_q(term + C::SLOTS)")
+    assert "stage_free()" in a[read:issue]
+    b = body["fast.cuh:k_col_b_tma"]
+    read, issue = b.index("qr[C::qat("), b.index("issue_q(term + 1)")
+    fence = b.find("fence_proxy_async()", read)
+    assert read < fence < b.index("__syncthreads_and(good)", read) < issue
