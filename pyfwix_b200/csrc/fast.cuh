@@ -800,10 +800,7 @@ __device__ __forceinline__ void kpow_factors(const SpecArgs& a, int t, int iw, i
   const KPow k(a, t, iw, x);
   if (k.n == 1) {  // the usual order, without the power loop
 #pragma unroll
-    for (int e = 0; e < P::E; ++e) {
-      const float ky = (float)fold_last<P>(lane_t, e) * k.dk;
-      f[e] = (k.kx2 + ky * ky) * k.s;
-    }
+    for (int e = 0; e < P::E; ++e) f[e] = k.ratio(fold_last<P>(lane_t, e)) * k.norm;
   } else {
 #pragma unroll
     for (int e = 0; e < P::E; ++e) f[e] = k.at(pos_last<P>(lane_t, e));

@@ -254,28 +254,33 @@ __device__ __forceinline__ float2 qmult(const SpecArgs& a, int t, int iw, int x,
 }
 
 // Born filter (|k| / w)^(2n) x norm of term t (order n = t + term0) along a column
-// (fixed x): a real factor, k^2n by products and norm / w^2n once per column, so a
-// sample takes four instructions instead of two table loads, a division and a
-// complex product (the scattering's column passes at 256 x 256 x 128: 71 -> 54 us
-// forward, 68 -> 57 adjoint, of floors of 31 and 20).  |ky| = |index| dk as in the wavenumber table.
+// (fixed x): a real factor, norm r^n of the ratio r = (kx^2 + ky^2) / w^2 with kx^2 / w^2
+// and dk^2 / w^2 formed once per column, so a sample takes five instructions instead of
+// two table loads, a division and a complex product (the scattering's column passes at
+// 256 x 256 x 128: 71 -> 54 us forward, 68 -> 57 adjoint, of floors of 31 and 20).  The power is
+// taken of the ratio, of order one up to the propagating limit in any unit: k^2n and
+// w^2n by themselves leave the range of a float from n = 3 on (at 20 kHz w^8 is 6e40).
+// |ky| = |index| dk as in the wavenumber table.
 struct KPow {
-  float kx2, dk, s;
+  float kx2, dk2, norm;  // kx^2 / w^2, dk^2 / w^2
   int n, NY;
   __device__ __forceinline__ KPow(const SpecArgs& a, int t, int iw, int x) {
-    const float kx = a.kx[x];
-    kx2 = kx * kx;
-    dk = a.d.NY > 1 ? a.ky[1] : 0.f;
+    const float kx = a.kx[x], dk = a.d.NY > 1 ? a.ky[1] : 0.f, w2 = a.w2[iw];
+    kx2 = kx * kx / w2;
+    dk2 = dk * dk / w2;
+    norm = a.norm;
     NY = a.d.NY;
     n = t + a.term0;
-    s = a.norm;
-    for (int k = 0; k < n; ++k) s /= a.w2[iw];
+  }
+  __device__ __forceinline__ float ratio(int ky) const {  // at folded row ky = min(y, NY - y)
+    const float i = (float)ky;
+    return fmaf(i * i, dk2, kx2);
   }
   __device__ __forceinline__ float at(int y) const {
-    const float ky = (float)min(y, NY - y) * dk;
-    const float k2 = kx2 + ky * ky;
-    float p = n == 0 ? 1.f : k2;
-    for (int k = 1; k < n; ++k) p *= k2;
-    return p * s;
+    const float r = ratio(min(y, NY - y));
+    float p = n == 0 ? 1.f : r;
+    for (int k = 1; k < n; ++k) p *= r;
+    return p * norm;
   }
 };
 
