@@ -397,7 +397,7 @@ __global__ void __launch_bounds__(kWarps * 32, row_fwd_min_blocks<P, PRE>()) k_r
   }
   constexpr bool kSmooth = PRE == W_SMOOTH_CONJ;
   __shared__ typename std::conditional<kSmooth, HatTables, int>::type hat;
-  float unit = 0.f;
+  PhaseUnit unit = {0.f, 0.f};
   if constexpr (kSmooth) {
     unit = phase_unit(a, c.iw);
     stage_hat(hat, a, c.iw, unit);
@@ -557,7 +557,7 @@ __global__ void __launch_bounds__(kWarps * 32, multi_term(POST) && (P::E == 16 |
   constexpr bool kPair = POST == W_SMOOTH_PAIR, kDeriv = kPair || POST == W_SMOOTH_DERIV;
   constexpr bool kSmooth = POST == W_SMOOTH || kDeriv;
   __shared__ typename std::conditional<kSmooth, HatTables, int>::type hat;
-  float unit = 0.f;
+  PhaseUnit unit = {0.f, 0.f};
   if constexpr (kSmooth) {
     unit = phase_unit(a, c.iw);
     stage_hat(hat, a, c.iw, unit);

@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(S::ROW_THREADS, min_blocks<S>(S::ROW_THREADS, 
   chain_wait();
   constexpr bool kSmooth = CLS == C_SMOOTH;
   __shared__ typename std::conditional<kSmooth, HatTables, int>::type hat;
-  float unit = 0.f;
+  PhaseUnit unit = {0.f, 0.f};
   if constexpr (kSmooth) {
     unit = phase_unit(a, c.iw);
     stage_hat(hat, a, c.iw, unit);
@@ -462,7 +462,7 @@ __global__ void __launch_bounds__(S::ROW_THREADS, min_blocks<S>(S::ROW_THREADS, 
   // kDeriv: the sum of w_r' C_r T_r beside the step's own
   constexpr bool kDeriv = CLS == C_PAIR || CLS == C_DERIV, kSmooth = CLS == C_SMOOTH || kDeriv;
   __shared__ typename std::conditional<kSmooth, HatTables, int>::type hat;
-  float unit = 0.f;
+  PhaseUnit unit = {0.f, 0.f};
   if constexpr (kSmooth) {
     unit = phase_unit(a, c.iw);
     stage_hat(hat, a, c.iw, unit);
