@@ -443,20 +443,21 @@ __global__ void __launch_bounds__(kWarps * 32, row_fwd_min_blocks<P, PRE>()) k_r
 #pragma unroll
     for (int e = 0; e < P::E; ++e) lab.set(e, c.live ? lrow[pos_first<P>(c.t, e)] : 255u);
   }
-  // smooth weights: each cell's fractional reference index and the cell part
+  // smooth weights: each cell's place between the references and the cell part
   // conj(B(s)) of every reference's weight, once per cell; terms that no sample of
   // the warp's rows supports are zero rows
   unsigned used = 0xffffffffu;
-  float g[kSmooth ? P::E : 1];
+  HatCells<kSmooth ? P::E : 1> hc;
   if constexpr (kSmooth) {
     const float* srow = a.sm_s + (long long)(c.live ? c.y : 0) * P::N;
     unsigned mine = 0;
 #pragma unroll
     for (int e = 0; e < P::E; ++e) {
       const float sv = c.live ? srow[pos_first<P>(c.t, e)] : 0.f;
-      g[e] = hat_index(hat, a.sm_n, sv);
+      const HatPos hp = hat_pos(hat, a.sm_n, sv);
+      hc.set(e, hp);
       if (c.live) {
-        mine |= hat_index_support(a.sm_n, g[e]);
+        mine |= hat_support(a.sm_n, hp.j);
         raw[e] = cmul_conj(raw[e], smooth_cell_phase(unit, sv));
       }
     }
@@ -479,7 +480,7 @@ __global__ void __launch_bounds__(kWarps * 32, row_fwd_min_blocks<P, PRE>()) k_r
     if constexpr (kSmooth) {
       const float2 C = hat.C[term];
 #pragma unroll
-      for (int e = 0; e < P::E; ++e) v[e] = cmul_conj(cscale(raw[e], hat_w(g[e], term)), C);  // raw is 0 where !live
+      for (int e = 0; e < P::E; ++e) v[e] = cmul_conj(cscale(raw[e], hc.w(e, term)), C);  // raw is 0 where !live
     } else if (kScatC && scat_smem) {
       const float f = 0.5f * a.w[c.iw] * a.dz * a.coef[term + a.term0];
       const float2* wrow = wt + ((size_t)term * RowGeo<P>::ROWS + (c.y - y0)) * P::N;
@@ -563,7 +564,7 @@ __global__ void __launch_bounds__(kWarps * 32, multi_term(POST) && (P::E == 16 |
     stage_hat(hat, a, c.iw, unit);
   }
   __syncthreads();
-  float g[kSmooth ? P::E : 1];
+  HatCells<kSmooth ? P::E : 1> hc;
   float2 acc[P::E];
   float2 acc2[kDeriv ? P::E : 1];
 #pragma unroll
@@ -593,8 +594,9 @@ __global__ void __launch_bounds__(kWarps * 32, multi_term(POST) && (P::E == 16 |
     const float* srow = a.sm_s + (long long)(c.live ? c.y : 0) * P::N;
 #pragma unroll
     for (int e = 0; e < P::E; ++e) {
-      g[e] = hat_index(hat, a.sm_n, c.live ? srow[pos_first<P>(c.t, e)] : 0.f);
-      if (c.live) mine |= hat_index_support(a.sm_n, g[e]);
+      const HatPos hp = hat_pos(hat, a.sm_n, c.live ? srow[pos_first<P>(c.t, e)] : 0.f);
+      hc.set(e, hp);
+      if (c.live) mine |= hat_support(a.sm_n, hp.j);
     }
     used = __reduce_or_sync(0xffffffffu, mine);
   }
@@ -634,12 +636,12 @@ __global__ void __launch_bounds__(kWarps * 32, multi_term(POST) && (P::E == 16 |
     if constexpr (kSmooth) {
       // reference part of the weights here, the cell part B(s) once after the sum
       const float2 C = hat.C[term];
-      const float below = hat.inv[term > 0 ? term - 1 : 0], above = hat.inv[term];
+      const float below = term > 0 ? hat.inv[term - 1] : 0.f, above = hat.inv[term];
 #pragma unroll
       for (int e = 0; e < P::E; ++e) {
         const float2 u = cmul(v[e], C);
-        acc[e] = cfma(u, hat_w(g[e], term), acc[e]);
-        if constexpr (kDeriv) acc2[e] = cfma(u, hat_dw(g[e], term, a.sm_n, below, above), acc2[e]);
+        acc[e] = cfma(u, hc.w(e, term), acc[e]);
+        if constexpr (kDeriv) acc2[e] = cfma(u, hc.dw(e, term, below, above), acc2[e]);
       }
     } else if (kScat && scat_smem) {
       if (!wt_ready) {  // every warp reaches this after its first transform (no term is skipped)

@@ -368,18 +368,19 @@ __global__ void __launch_bounds__(S::ROW_THREADS, min_blocks<S>(S::ROW_THREADS, 
   } else {
     __syncthreads();
   }
-  // smooth weights: a cell's fractional reference index, and the cell part conj(B(s))
+  // smooth weights: a cell's place between the references, and the cell part conj(B(s))
   // of every reference's weight once per cell
-  float hg[kSmooth ? RT : 1];
+  HatCells<kSmooth ? RT : 1> hc;
   if constexpr (kSmooth) {
     unsigned mine = 0;
     const float* srow = a.sm_s + (long long)(c.live ? c.y : 0) * d.n();
 #pragma unroll
     for (int r = 0; r < RT; ++r) {
       const float sv = c.live ? srow[c.j + r * d.nt()] : 0.f;
-      hg[r] = hat_index(hat, a.sm_n, sv);
+      const HatPos hp = hat_pos(hat, a.sm_n, sv);
+      hc.set(r, hp);
       if (c.live) {
-        mine |= hat_index_support(a.sm_n, hg[r]);
+        mine |= hat_support(a.sm_n, hp.j);
         raw[r] = cmul_conj(raw[r], smooth_cell_phase(unit, sv));
       }
     }
@@ -408,7 +409,7 @@ __global__ void __launch_bounds__(S::ROW_THREADS, min_blocks<S>(S::ROW_THREADS, 
       } else if constexpr (kSmooth) {
         const float2 C = hat.C[term];
 #pragma unroll
-        for (int r = 0; r < RT; ++r) v[r] = cmul_conj(cscale(raw[r], hat_w(hg[r], term)), C);
+        for (int r = 0; r < RT; ++r) v[r] = cmul_conj(cscale(raw[r], hc.w(r, term)), C);
       } else {
 #pragma unroll
         for (int r = 0; r < RT; ++r) v[r] = raw[r];
@@ -489,14 +490,15 @@ __global__ void __launch_bounds__(S::ROW_THREADS, min_blocks<S>(S::ROW_THREADS, 
   } else {
     __syncthreads();
   }
-  float hg[kSmooth ? RT : 1];
+  HatCells<kSmooth ? RT : 1> hc;
   if constexpr (kSmooth) {
     unsigned mine = 0;
     const float* srow = a.sm_s + (long long)(c.live ? c.y : 0) * d.n();
 #pragma unroll
     for (int r = 0; r < RT; ++r) {
-      hg[r] = hat_index(hat, a.sm_n, c.live ? srow[c.j + r * d.nt()] : 0.f);
-      if (c.live) mine |= hat_index_support(a.sm_n, hg[r]);
+      const HatPos hp = hat_pos(hat, a.sm_n, c.live ? srow[c.j + r * d.nt()] : 0.f);
+      hc.set(r, hp);
+      if (c.live) mine |= hat_support(a.sm_n, hp.j);
     }
     used = cta_or(mine);
   }
@@ -545,12 +547,12 @@ __global__ void __launch_bounds__(S::ROW_THREADS, min_blocks<S>(S::ROW_THREADS, 
     } else if constexpr (kSmooth) {
       // reference part of the weights here, the cell part B(s) once after the sum
       const float2 C = hat.C[term];
-      const float below = hat.inv[term > 0 ? term - 1 : 0], above = hat.inv[term];
+      const float below = term > 0 ? hat.inv[term - 1] : 0.f, above = hat.inv[term];
 #pragma unroll
       for (int r = 0; r < RT; ++r) {
         const float2 u = cmul(v[r], C);
-        acc[r] = cfma(u, hat_w(hg[r], term), acc[r]);
-        if constexpr (kDeriv) acc2[r] = cfma(u, hat_dw(hg[r], term, a.sm_n, below, above), acc2[r]);
+        acc[r] = cfma(u, hc.w(r, term), acc[r]);
+        if constexpr (kDeriv) acc2[r] = cfma(u, hc.dw(r, term, below, above), acc2[r]);
       }
     } else {
 #pragma unroll

@@ -84,23 +84,12 @@ __device__ __forceinline__ Hat hat_weight(const float* ref, int n, int t, float 
   return h;
 }
 
-// Terms whose hat weight or its derivative can be nonzero at slowness s (bit r
-// for reference r; only the bracketing pair, or one end reference outside).
-__device__ __forceinline__ unsigned hat_support(const float* ref, int n, float s) {
-  if (n == 1 || s <= ref[0]) return 1u;
-  if (s >= ref[n - 1]) return 1u << (n - 1);
-  int j = 0;
-  while (j < n - 2 && s >= ref[j + 1]) ++j;
-  return 3u << j;
-}
-
 // The split-step factor of the smooth step factors into a cell part and a
 // reference part: SS_r = exp(-i w (s - s_r) dz) = B(s) C_r with B(s) =
 // exp(-i w s dz) and C_r = exp(i w s_r dz).  The register-resident row passes
 // take one sine / cosine per cell (B, applied once to the sum over references, or
 // once to the input of the adjoint) and one per reference and CTA (C_r, in shared
-// memory).  The hat weight of reference t is max(0, 1 - |g - t|) at a cell's
-// fractional reference index g, a real factor of t's transform, and the
+// memory).  The hat weight of reference t is a real factor of t's transform, and the
 // derivative (w_r' - i w dz w_r) SS_r needs only the sum S1 of w_r' C_r T_r beside
 // the step's own sum S of w_r C_r T_r: it is (S1 - i w dz S) B.  (With a complex
 // weight per cell and term, sines of C_r in every lane and branches for the hat the
@@ -145,32 +134,50 @@ __device__ __forceinline__ void stage_hat(HatTables& h, const SpecArgs& a, int i
 __device__ __forceinline__ float2 smooth_cell_phase(PhaseUnit unit, float s) {  // B(s)
   return cconj(phase_factor(unit, s));
 }
-// Fractional reference index g of slowness s: the hat weights are 1 - (g - j) on
-// reference j and g - j on j + 1, j = min(floor g, n - 2); g = 0 and g = n - 1 are
-// the clamped ends (weight 1 on the end reference, derivative 0).  Same
-// bracketing as hat_weight.
-__device__ __forceinline__ float hat_index(const HatTables& h, int n, float s) {
-  if (n == 1 || s <= h.ref[0]) return 0.f;
-  if (s >= h.ref[n - 1]) return (float)(n - 1);
+// Where a slowness s lies between the references: the hat weights are 1 - u on
+// reference j and u on j + 1, those of hat_weight with the same rounding.  At and
+// beyond the last reference j = n - 1, u = 0; at and below the first j = kBelow (one
+// below zero in the bytes that hold j), u = 1: weight 1 on the end reference, and the
+// derivative's factors are 0 there (HatTables::inv, hat_dw).
+constexpr unsigned kBelow = 255;  // nref is at most 255
+struct HatPos {
+  unsigned j;
+  float u;
+};
+__device__ __forceinline__ HatPos hat_pos(const HatTables& h, int n, float s) {
+  if (n == 1) return {0u, 0.f};
+  if (s <= h.ref[0]) return {kBelow, 1.f};
+  if (s >= h.ref[n - 1]) return {(unsigned)(n - 1), 0.f};
   int j = 0;
   for (int k = 1; k < n - 1; ++k) j += s >= h.ref[k] ? 1 : 0;
-  return (float)j + (s - h.ref[j]) * h.inv[j];
+  return {(unsigned)j, (s - h.ref[j]) / (h.ref[j + 1] - h.ref[j])};
 }
-// Terms that index g gives a weight or derivative (n <= 32; every bit beyond).
-__device__ __forceinline__ unsigned hat_index_support(int n, float g) {
-  if (n > 32) return 0xffffffffu;
-  if (n == 1 || g <= 0.f) return 1u;
-  if (g >= (float)(n - 1)) return 1u << (n - 1);
-  return 3u << min((int)g, n - 2);
+// Terms that a cell in interval j gives a weight or derivative (n <= 32; every bit beyond).
+__device__ __forceinline__ unsigned hat_support(int n, unsigned j) {
+  return n > 32 ? 0xffffffffu : j == kBelow ? 1u : 3u << j;
 }
-__device__ __forceinline__ float hat_w(float g, int t) { return __saturatef(1.f - fabsf(g - (float)t)); }
-// Slowness derivative of reference t's weight (interval j = floor g: -inv[j] on j,
-// inv[j] on j + 1).
-__device__ __forceinline__ float hat_dw(float g, int t, int n, float inv_below, float inv_above) {
-  const float d = g - (float)t;
-  const float v = d >= 0.f ? (d < 1.f ? -inv_above : 0.f) : (d >= -1.f ? inv_below : 0.f);
-  return g > 0.f && g < (float)(n - 1) ? v : 0.f;
-}
+// The positions of a thread's N cells, the intervals as bytes.  (Interval and fraction
+// in one float, j + u, lose the fraction's last bits to the interval's: from j = 128 on
+// a weight has 16 of its 24.)
+template <int N>
+struct HatCells {
+  float u[N];
+  unsigned j4[(N + 3) / 4];
+  __device__ __forceinline__ void set(int i, HatPos p) {
+    u[i] = p.u;
+    j4[i / 4] = i % 4 ? j4[i / 4] | p.j << 8 * (i % 4) : p.j;
+  }
+  // Weight of reference t at cell i (real factor of t's transform).
+  __device__ __forceinline__ float w(int i, unsigned t) const {
+    const unsigned j = j4[i / 4] >> 8 * (i % 4) & 255u;
+    return j == t ? 1.f - u[i] : j == (t - 1 & 255u) ? u[i] : 0.f;
+  }
+  // Its slowness derivative: -above on reference j, below on j + 1.
+  __device__ __forceinline__ float dw(int i, unsigned t, float below, float above) const {
+    const unsigned j = j4[i / 4] >> 8 * (i % 4) & 255u;
+    return j == t ? -above : j == (t - 1 & 255u) ? below : 0.f;
+  }
+};
 
 // w_r SS_r (W_SMOOTH), w_r conj(SS_r) (W_SMOOTH_CONJ) or (w_r' - i w dz w_r) SS_r
 // (W_SMOOTH_DERIV) for reference t at cell (y, x) of frequency iw.

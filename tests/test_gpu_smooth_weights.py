@@ -22,13 +22,14 @@ TOL = 2.1e-7
 SIZES = [(256, 20), (50, 45), (147, 24), (15, 30)]
 
 
-def _case(nx, ny, n, dz, fmax):
+def _case(nx, ny, n, dz, fmax, clamped=True):
     rng = np.random.default_rng(n + nx)
     lo, hi = 1.0 / 2200.0, 1.0 / 1500.0
     refs = np.linspace(lo, hi, n).astype(np.float32) if n > 1 else np.array([lo], np.float32)
     s = rng.uniform(lo, hi, (ny, nx)).astype(np.float32)
-    # clamped cells, cells on a reference and one step below and above it
-    s.flat[0::7] = rng.choice([0.9 * lo, 1.1 * hi], s.flat[0::7].size).astype(np.float32)
+    # clamped cells; cells on a reference and one step below and above it
+    if clamped:
+        s.flat[0::7] = rng.choice([0.9 * lo, 1.1 * hi], s.flat[0::7].size).astype(np.float32)
     s.flat[1::7] = rng.choice(refs, s.flat[1::7].size)
     s.flat[2::7] = np.nextafter(rng.choice(refs, s.flat[2::7].size), np.float32(0))
     s.flat[3::7] = np.nextafter(rng.choice(refs, s.flat[3::7].size), np.float32(1))
@@ -66,10 +67,8 @@ CASES = [(1, 10.0, 40.0), (4, 10.0, 40.0), (4, 50.0, 100.0), (32, 10.0, 40.0), (
          (200, 10.0, 40.0)]
 
 
-@pytest.mark.parametrize("nx,ny", SIZES)
-@pytest.mark.parametrize("n,dz,fmax", CASES)
-def test_forward_and_derivative(nx, ny, n, dz, fmax):
-    p, refs, s, w, x = _case(nx, ny, n, dz, fmax)
+def _forward_and_derivative(case, n, dz):
+    p, refs, s, w, x = case
     wt, dw = _hat(refs, s)
     wdz = (w * dz)[None, :, None, None]
     want, wder, mag = 0, 0, 0
@@ -86,6 +85,22 @@ def test_forward_and_derivative(nx, ny, n, dz, fmax):
     p.smooth_step_pair(n, to_dev(x), out, der)
     assert rel(to_host(out), want) < TOL
     assert np.linalg.norm(to_host(der) - wder) < TOL * np.linalg.norm(mag)
+
+
+@pytest.mark.parametrize("nx,ny", SIZES)
+@pytest.mark.parametrize("n,dz,fmax", CASES)
+def test_forward_and_derivative(nx, ny, n, dz, fmax):
+    _forward_and_derivative(_case(nx, ny, n, dz, fmax), n, dz)
+
+
+@pytest.mark.parametrize("nx,ny", SIZES)
+@pytest.mark.parametrize("n", [128, 255])
+def test_every_bit_of_the_weights(nx, ny, n):
+    """Many references on steps of 2 km, so that neighbouring ones give transforms a radian or
+    two apart and a weight's error is not cancelled by its neighbour's.  (Beside the
+    roundings above only that of the frequency, 0.6 u of a bracket's 2 radians at most:
+    the same bound.  No cells beyond the references: those are 60 radians away.)"""
+    _forward_and_derivative(_case(nx, ny, n, 2000.0, 100.0, clamped=False), n, 2000.0)
 
 
 @pytest.mark.parametrize("nx,ny", SIZES)
