@@ -46,6 +46,7 @@ import warnings
 
 import numpy as np
 import torch
+from torch.autograd import forward_ad
 
 from . import _lib as L
 from . import hostcopy, refsampler
@@ -121,13 +122,18 @@ def _dev(x, device, shape=None, zero=False):
 def _out(x, device, src):
     """Device tensor for a result that the operator writes in full, computed from the
     device tensor ``src``: the operand itself where it is one, without the zero fill
-    of a sum (a launch and a pass over the field).  An operand that shares its memory
-    with ``src``, or is not of its size, is zeroed first, as a sum's would be."""
+    of a sum (a launch and a pass over the field).  An operand that shares memory with
+    ``src``, or is not of its size, is zeroed first, as a sum's would be; so is one that
+    autograd follows (grad, forward mode, inference), since the fill is what refuses or
+    records the write.  Without the fill the write is still counted as one in place, so
+    that a tensor saved for a backward pass is seen to have changed."""
     t = _raw(x)
-    if (isinstance(t, torch.Tensor) and t.device == device and t.dtype == torch.complex64 and t.is_contiguous()
-            and t.numel() == src.numel()
-            and t.untyped_storage().data_ptr() != src.untyped_storage().data_ptr()):
-        return t
+    if (type(t) is torch.Tensor and t.device == device and t.dtype == torch.complex64 and t.is_contiguous()
+            and t.numel() == src.numel() and not (t.requires_grad or t.is_inference() or forward_ad._current_level >= 0)):
+        n, a, b = 8 * t.numel(), t.data_ptr(), src.data_ptr()
+        if a + n <= b or b + n <= a:
+            torch.autograd.graph.increment_version(t)
+            return t
     return _dev(x, device, zero=True)
 
 
