@@ -607,9 +607,10 @@ __global__ void __launch_bounds__(kWarps * 32, multi_term(POST) && (P::E == 16 |
   };
   const long long roff = (c.bl * a.d.NY + (c.live ? c.y : 0)) * P::N;
   int term = next_term(0);
-  // the next term's row is prefetched, except where the paired sums of 16-sample
-  // lanes leave no registers for it (two accumulators, the term and the hat indices)
-  constexpr bool kPrefetch = FWIX_ROWINV_PREFETCH && !(kDeriv && P::E >= 16);
+  // the next term's row is prefetched, except where the smooth weights leave no registers
+  // for it (accumulators, the term and the hat positions: the step on 256 x 256 x 64 with
+  // twelve references 309 us with it, 289 without)
+  constexpr bool kPrefetch = FWIX_ROWINV_PREFETCH && !kSmooth;
   float2 pre[kPrefetch ? P::E : 1];
   if (kPrefetch && term < nterm) {
     const float2* src = a.t2 + (long long)term * a.tstride + roff;
