@@ -340,9 +340,9 @@ struct RowCtx {
   }
 };
 
-// Resident CTAs per SM the forward row pass's registers are held to: the
-// multi-term passes of 12- and 16-sample lanes at two (the scattering adjoint's,
-// with one term's weights and no labels, at three), the rest unhinted.
+// Resident CTAs per SM the forward row pass's registers are held to (rows are compiled
+// for 16-sample lanes only): the multi-term passes at two (the scattering adjoint's, with
+// one term's weights and no labels, at three), the rest unhinted.
 // Compile-time occupancy knobs (defaults as measured best): resident CTAs of the
 // multi-term forward and inverse row passes and of the multi-input and the
 // single-input column pass with 16-sample lanes, and whether the multi-term
@@ -361,8 +361,8 @@ struct RowCtx {
 #endif
 template <class P, int PRE>
 constexpr int row_fwd_min_blocks() {
-  if (PRE == W_SCAT_CONJ && P::E == 16) return 3;
-  return multi_term(PRE) && (P::E == 16 || P::E == 12) ? FWIX_ROW_MULTI_MINB : 0;
+  if (PRE == W_SCAT_CONJ) return 3;
+  return multi_term(PRE) ? FWIX_ROW_MULTI_MINB : 0;
 }
 
 // t1[term] = F_x(pre_term * in) for each term.  RF: the input is in + the
@@ -516,8 +516,7 @@ __global__ void __launch_bounds__(kWarps * 32, row_fwd_min_blocks<P, PRE>()) k_r
 // reflection terms of SpecArgs::rf_at 2 (separate instances, as in the forward
 // row pass).
 template <class P, int POST, bool RF = false>
-__global__ void __launch_bounds__(kWarps * 32, multi_term(POST) && (P::E == 16 || P::E == 12) ? FWIX_ROW_MULTI_MINB
-                                                                                              : (RF && POST == W_ONE ? 4 : 0))
+__global__ void __launch_bounds__(kWarps * 32, multi_term(POST) ? FWIX_ROW_MULTI_MINB : (RF && POST == W_ONE ? 4 : 0))
     k_row_inv(const SpecArgs a, int nchunk, int post_taper) {
   extern __shared__ float2 smem[];
   RowCtx<P> c(a, smem, nchunk);
