@@ -91,14 +91,20 @@ __global__ void __launch_bounds__(kCells * kGroups)
   if (!c.ok) return;
   float2 r = mw == 0 ? rs[threadIdx.x] : make_float2(0.f, 0.f);
   const int ns = S1 ? 1 : d.ns;
-#pragma unroll 4
+  // Not unrolled: the warps hide each other's loads, and few registers let all of them in.
+  // The first shot's samples are fetched ahead of the coefficient's roots.  (256 x 256 x
+  // 128: a model per frequency 121 us unrolled by four, 94 so; one model 53 and 45.)
+#pragma unroll 1
   for (int iw = threadIdx.y; iw < d.nw; iw += kGroups) {
+    const long long k0 = wf_index(d, 0, iw, c);
+    const float2 v0 = in[k0], o0 = out[k0];
     if (mw != 0) {
       const long long m = iw * mw + c.yx;
       r = refl_coef(s0[m], s1[m], r0[m], r1[m]);
       if (adjoint) r = cconj(r);
     }
-    for (int s = 0; s < ns; ++s) {
+    out[k0] = cadd(o0, cmul(v0, r));
+    for (int s = 1; s < ns; ++s) {
       const long long k = wf_index(d, s, iw, c);
       out[k] = cadd(out[k], cmul(in[k], r));
     }
