@@ -1003,7 +1003,11 @@ __device__ __forceinline__ bool qflip(const SpecArgs& a, int t, int iw) {
 // Resident CTAs a TMA column pass is held to: what its shared memory lets an SM hold,
 // as far as its registers go: two for 12 samples per lane and more (three for the
 // single-input pass of 16 without phase tiles; 12 at three spilled 180 - 260 bytes in
-// the multi-input pass, 314 -> 339 us at 384 x 384 x 96), four for 8.
+// the multi-input pass, 314 -> 339 us at 384 x 384 x 96), four for 8.  20 samples without
+// phase tiles spill 70 - 330 bytes at two and are still faster than at one without spills,
+// us of the single- and the multi-input pass with four references: 320 x 320 x 64 evaluated
+// in the kernel 302 and 326 at two, 394 and 426 at one; 270 x 320 x 64 from the table 125 and
+// 136, 146 and 166; 320 x 640 x 32 evaluated 356 and 430, 493 and 496.
 template <class P>
 constexpr int col_tma_min_blocks(bool qtile, bool single) {
   const int fit = qtile ? ColTma<P>::fit(ColTma<P>::SLOTS)

@@ -157,20 +157,26 @@ struct SpecArgs {
 // pointers, never const __restrict__: that promises memory which no one writes while
 // the kernel runs, so its loads may go to the non-coherent read-only path or ahead of
 // chain_wait(), and here the kernel before still writes while this one starts.  (An
-// output that the kernel itself writes may be __restrict__.)  The prologue and the launch gap (1 - 2 us of kernels of
-// 5 - 30 us at 128 x 128 and below) then go under the kernel before: modelling at 128
-// x 128 x 64 2432 -> 2042 us, the Born pair at 256 x 256 x 128 13.71 -> 13.35 ms.  A grid
-// of more than a wave calls chain_next() at its start (SpecArgs::early; at the last
-// stage instead the Born pair takes 12.75 ms for 12.46), a smaller one at its last
-// stage: CTAs placed early fill the SMs that run dry first, and the next grid, of less
-// than a wave too, would run on a part of the GPU (NSPS step and adjoint at 105 x 90 x
-// 24, queued back to back, 54.7 us early and 39.1 late).  Instances that share the
-// GPU over several streams are not chained (fwix_sweep): there the waiting CTAs hold
-// places that the other streams' kernels could use (6.31 -> 6.48 ms, four shots).
+// output that the kernel itself writes may be __restrict__.)
+//
+// The prologue and the launch gap (1 - 2 us of kernels of 5 - 30 us at 128 x 128 and below)
+// then go under the kernel before: modelling at 128 x 128 x 64 2432 -> 2042 us, the Born
+// pair at 256 x 256 x 128 13.71 -> 13.35 ms.  A grid of more than a wave calls chain_next()
+// at its start (SpecArgs::early; at the last stage instead the Born pair takes 12.75 ms
+// for 12.46), a smaller one at its last stage: CTAs placed early fill the SMs that run dry
+// first, and the next grid, of less than a wave too, would run on a part of the GPU (NSPS
+// step and adjoint at 105 x 90 x 24, queued back to back, 54.7 us early and 39.1 late).
+//
+// A batch that fwix_sweep puts on several streams is not chained: its streams are full, and
+// the waiting CTAs hold places that the other streams' kernels could use (6.31 -> 6.48
+// ms, four shots).  Windows on a stream each (streaming.py) are: the host enqueues
+// them one after the other, and the streams overlap little (two groups x two bands of 240 x
+// 200 x 48 3.92 ms unchained and 3.68 chained, their Born pair 6.5 and 5.8; on 480 x 400 x
+// 64, where the GPU is full, 10.87 and 10.95, Born 33.3 and 33.4).
 #ifdef __CUDACC__
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// chain_next() for a grid of plain threads that exceeds what the SMs hold at once.
+// chain_next() for a grid of plain threads that exceeds what the 148 SMs hold at once.
 __device__ __forceinline__ void chain_next_if_large() {
   if (gridDim.x * gridDim.y > 148u * (2048u / (blockDim.x * blockDim.y))) chain_next();
 }

@@ -91,10 +91,11 @@ __device__ __forceinline__ Hat hat_weight(const float* ref, int n, int t, float 
 // once to the input of the adjoint) and one per reference and CTA (C_r, in shared
 // memory).  The hat weight of reference t is a real factor of t's transform, and the
 // derivative (w_r' - i w dz w_r) SS_r needs only the sum S1 of w_r' C_r T_r beside
-// the step's own sum S of w_r C_r T_r: it is (S1 - i w dz S) B.  (With a complex
-// weight per cell and term, sines of C_r in every lane and branches for the hat the
-// 384 x 384 x 96 inverse row passes took 373 us (step), 395 (derivative) and 476
-// (both) and the forward one 323; now 293, 312, 324 and 249.)
+// the step's own sum S of w_r C_r T_r: it is (S1 - i w dz S) B.  (Steps at 384 x 384 x 96
+// with four references, with a complex weight per cell and term, sines of C_r in every lane
+// and branches for the hat: 732 us forward, 725 adjoint, 761 derivative, 871 both; so and
+// with flex.cuh's rows 576, 567, 610 and 622.  At 256 x 256 x 128, on the same rows, 348, 328,
+// 364 and 402; now 300, 266, 331 and 339.)
 constexpr int kMaxRefs = 256;  // more than a plan can have
 struct HatTables {
   float ref[kMaxRefs];
