@@ -1243,10 +1243,15 @@ __global__ void __launch_bounds__(kWarps * 32, col_tma_min_blocks<P>(kQT, true))
       tma::store_commit();
     }
   };
-  // The previous store has read the staging tile; every lane's phase reads precede
-  // the load that takes their slot next (the fence: they went by the generic proxy).
+  // The next phase tile takes a slot that every lane has read by the generic proxy: past a
+  // proxy fence and a barrier, that is behind the term's store, or, with one slot, which
+  // the next term waits for, already with the staging tile's release, at a fence of its
+  // own (320 x 320 x 80 migration 6.60 ms so, 6.79 behind the store; with two slots the
+  // extra fence costs modelling at 128 x 128 x 64 1.87 ms for 1.85).
+  constexpr bool kEarlyQ = kQT && C::SLOTS == 1;
+  // The previous store has read the staging tile.
   auto stage_free = [&]() {
-    if constexpr (kQT) tma::fence_proxy_async();
+    if constexpr (kEarlyQ) tma::fence_proxy_async();
     if (threadIdx.x == 0) tma::store_wait_read();
     __syncthreads();
   };
@@ -1290,12 +1295,15 @@ __global__ void __launch_bounds__(kWarps * 32, col_tma_min_blocks<P>(kQT, true))
     if (term + 1 == nterm) chain_next();
     fft_inv<P>(v, t, tw, line);
     stage_free();
-    if constexpr (kQT) {  // every lane has read this term's factors
+    if constexpr (kEarlyQ) {
       if (threadIdx.x == 0) issue_q(term + C::SLOTS);
     }
 #pragma unroll
     for (int e = 0; e < P::E; ++e) stage[tma::swz_tile<C::LX>(pos_first<P>(t, e), col)] = v[e];
     store(term);
+    if constexpr (kQT && !kEarlyQ) {
+      if (threadIdx.x == 0) issue_q(term + C::SLOTS);
+    }
   }
   if (threadIdx.x == 0) tma::store_wait_read();
 }

@@ -84,6 +84,10 @@ def test_phase_slots_are_fenced_before_their_next_load():
     assert 0 <= free.find("fence_proxy_async()") < free.find("__syncthreads()")
     read, issue = a.index("qr[T::qat("), a.index("issue_q(term + C::SLOTS)")
     assert "stage_free()" in a[read:issue]
+    late = a.index("issue_q(term + C::SLOTS)", issue + 1)  # the other place: behind the store's fence and barrier
+    put = a[a.index("auto store ="):]
+    put = put[:put.index("};")]
+    assert 0 <= put.find("fence_proxy_async()") < put.find("__syncthreads()") and "store(term);" in a[issue:late]
     b = body["fast.cuh:k_col_b_tma"]
     read, issue = b.index("qr[C::qat("), b.index("issue_q(term + 1)")
     fence = b.find("fence_proxy_async()", read)
