@@ -478,7 +478,8 @@ __global__ void __launch_bounds__(256) k_phase_table(const SpecArgs a, int nblk,
   if (ks >= rows) return;
   dst += ks * nf;
   for (int kf = threadIdx.x % 32; kf < nf; kf += 32)
-    dst[kf] = qmult<Q_PS_FWD>(b, r, iw, ky_fast ? k0 + ks : kf, ky_fast ? kf : k0 + ks);
+    // (the ky extent is rounded up to even: a one-row grid has a column past its table)
+    dst[kf] = qmult<Q_PS_FWD>(b, r, iw, ky_fast ? k0 + ks : kf, min(ky_fast ? kf : k0 + ks, a.d.NY - 1));
 }
 
 cudaError_t launch_phase_table(const SpecArgs& a, float2* dst, cudaStream_t s) {

@@ -37,6 +37,17 @@ def test_steps(nx, ny, padx, pady, eps, nref):
             assert rel(y, adj(g, sref[1], lab[1], x, d0)) < TOL
 
 
+@pytest.mark.parametrize("nx,ny", [(64, 1), (50, 1), (1, 64), (1, 48), (1, 1)])
+def test_one_row_or_column(nx, ny):
+    g, rng, sref, labels, _, _ = make_case(nx=nx, ny=ny, nw=2, nz=1, nref=3, taperx=0, tapery=0)
+    lab, x = oracle_labels(labels, g), wavefield(rng, 1, g)
+    p = make_plan(g, 1, sref, labels)
+    for kind, fwd, adj in (("pspi", wem.pspi_forward, wem.pspi_adjoint), ("nsps", wem.nsps_forward, wem.nsps_adjoint)):
+        y = torch.empty(p.wshape, dtype=torch.complex64, device="cuda")
+        assert rel(to_host(p.step(0, to_dev(x), y, kind=kind)), fwd(g, sref[0], lab[0], x)) < TOL
+        assert rel(to_host(p.step(0, to_dev(x), y, kind=kind, direction=1)), adj(g, sref[0], lab[0], x)) < TOL
+
+
 @pytest.mark.parametrize("nx,ny,padx,pady", NEITHER)
 @pytest.mark.parametrize("taylor,shared", [(0, True), (1, True), (4, False)])
 def test_scatter(nx, ny, padx, pady, taylor, shared):
