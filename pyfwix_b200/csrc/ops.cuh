@@ -114,8 +114,9 @@ __device__ __forceinline__ PhaseUnit phase_unit(const SpecArgs& a, int iw) {
 // (cos, sin)(w s dz).  B and C_r carry the phase of the full w s dz, their product only
 // that of w (s - s_r) dz: the product u s is taken in two floats, its head through
 // sincospif (whose range reduction is exact) and its tail as a small rotation, so that
-// both keep their last bits at any phase (head only: 3.6e-7 of the step's result at
-// 100 Hz x 50 m, 21 radians; six instructions a cell).
+// both keep their last bits at any phase (of the step's result at 100 Hz x 50 m, 21 radians,
+// head only 3.6e-7, so 6.1e-8, and 4.3e-8 with a phase per cell and reference as in
+// spectral.cu; six instructions a cell).
 __device__ __forceinline__ float2 phase_factor(PhaseUnit u, float s) {
   const float p = u.hi * s;
   const float e = 3.14159265358979f * fmaf(u.lo, s, fmaf(u.hi, s, -p));
@@ -159,7 +160,8 @@ __device__ __forceinline__ unsigned hat_support(int n, unsigned j) {
 }
 // The positions of a thread's N cells, the intervals as bytes.  (Interval and fraction
 // in one float, j + u, lose the fraction's last bits to the interval's: from j = 128 on
-// a weight has 16 of its 24.)
+// a weight has 16 of its 24; of the result of a step of 2 km over 255 references 7.4e-7,
+// so 6.1e-8.)
 template <int N>
 struct HatCells {
   float u[N];
